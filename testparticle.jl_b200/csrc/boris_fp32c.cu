@@ -41,13 +41,10 @@ __device__ __forceinline__ bool outside32(const BorisArgs& a, const CPos& p, con
         const float x = p.hi[0] + p.lo[0], y = p.hi[1] + p.lo[1], z = p.hi[2] + p.lo[2];
         if (f & TP_TERM_SHELL) {
             const float r2 = fmaf(x, x, fmaf(y, y, z * z));
-            const float rmin2 = T.rmin > 0.0 ? (float)(T.rmin * T.rmin) : -1.0f;
-            const float rmax2 = T.rmax >= 0.0 ? (float)(T.rmax * T.rmax) : -1.0f;
-            if (r2 < rmin2 || r2 > rmax2) return true;
+            if (r2 < T.smin32 || r2 > T.smax32) return true;
         }
         if (f & TP_TERM_BOX) {
-            if (x < (float)T.lo[0] || x > (float)T.hi[0] || y < (float)T.lo[1] || y > (float)T.hi[1] ||
-                z < (float)T.lo[2] || z > (float)T.hi[2])
+            if (x < T.lo32[0] || x > T.hi32[0] || y < T.lo32[1] || y > T.hi32[1] || z < T.lo32[2] || z > T.hi32[2])
                 return true;
         }
     }

@@ -18,60 +18,9 @@
 //                                  with Boris (boris.jl:19-45) or
 //                                  Multistep (multistep_boris.jl:65-142) updates
 //   k_adaptive64<MULTI, QUEUE, FK> _adaptive_boris_single (adaptive_boris.jl:145-266)
-#include "fields64.cuh"
-#include "tp_launch.h"
+#include "boris64_common.cuh"
 
 namespace tpb {
-
-namespace {
-
-template <int FK>
-struct Saver64 {
-    const BorisArgs& a;
-    int W;
-    __device__ Saver64(const BorisArgs& a_)
-        : a(a_), W(6 + (a_.save_fields ? 6 : 0) + (a_.save_work ? 4 : 0)) {}
-    // slot k of particle i: state, then E and B at (r, t) when save_fields
-    // (_prepare_saved_data, boris.jl:405-440); the four work-rate columns of
-    // save_work are filled by a post-pass over the saved states
-    __device__ __forceinline__ void save(int64_t i, int64_t k, D3 r, D3 v, double t) const {
-        if (k >= a.nslots) {
-            set_status(a.status, TP_E_OVERFLOW);
-            return;
-        }
-        const int64_t n = a.n;
-        a.t_out[k * n + i] = t;
-        double* u = a.u_out + (k * W) * n + i;
-        u[0 * n] = r.x;
-        u[1 * n] = r.y;
-        u[2 * n] = r.z;
-        u[3 * n] = v.x;
-        u[4 * n] = v.y;
-        u[5 * n] = v.z;
-        if (a.save_fields) {
-            D3 E, B;
-            eval_EB64t<FK>(a.f, r, t, E, B);
-            u[6 * n] = E.x;
-            u[7 * n] = E.y;
-            u[8 * n] = E.z;
-            u[9 * n] = B.x;
-            u[10 * n] = B.y;
-            u[11 * n] = B.z;
-        }
-    }
-};
-
-template <bool QUEUE>
-__device__ __forceinline__ int64_t next_particle(const BorisArgs& a, int64_t& first) {
-    if (!QUEUE) {
-        int64_t g = first;
-        first = a.n;  // static: one particle per thread
-        return take_particle(a, g);
-    }
-    return take_particle(a, (int64_t)atomicAdd(a.queue, 1ULL));
-}
-
-}  // namespace
 
 // ---------------------------------------------------------------- fixed step
 template <bool MULTI, bool QUEUE, int FK>
@@ -472,13 +421,19 @@ __global__ void __launch_bounds__(TPB_ADAPTIVE64_BOUND(FK), 1) k_adaptive64(Bori
 template <bool MULTI, bool QUEUE, int FK>
 static const void* kernel_ptr64(bool adaptive, int ppt) {
     if (adaptive) return (const void*)k_adaptive64<MULTI, QUEUE, FK>;
-    if (FK == FK_ANALYTIC && ppt == 2) return (const void*)k_fixed64_slots<MULTI, QUEUE, FK, 2>;
+    if constexpr (FK == FK_ANALYTIC)
+        if (ppt == 2) return (const void*)k_fixed64_slots<MULTI, QUEUE, FK, 2>;
     return (const void*)k_fixed64<MULTI, QUEUE, FK>;
 }
 
 template <bool MULTI, bool QUEUE>
-static const void* pick_fk64(bool adaptive, int fk, int ppt) {
-    if (fk == FK_ANALYTIC) return kernel_ptr64<MULTI, QUEUE, FK_ANALYTIC>(adaptive, ppt);
+static const void* pick_fk64(bool adaptive, const BorisArgs& a) {
+    const int fk = kernel_config_of(a.f);
+    if (fk == FK_DIPOLE || fk == FK_UNIFORM) {
+        if (!adaptive && a.ppt != 2) return seg_kernel64(a, QUEUE);
+        return kernel_ptr64<MULTI, QUEUE, FK_ANALYTIC>(adaptive, a.ppt);
+    }
+    if (fk == FK_ANALYTIC) return kernel_ptr64<MULTI, QUEUE, FK_ANALYTIC>(adaptive, a.ppt);
     if (fk == FK_EBGRID) return kernel_ptr64<MULTI, QUEUE, FK_EBGRID>(adaptive, 1);
     if (fk == FK_GENGRID) return kernel_ptr64<MULTI, QUEUE, FK_GENGRID>(adaptive, 1);
     return kernel_ptr64<MULTI, QUEUE, FK_GENERIC>(adaptive, 1);
@@ -487,10 +442,8 @@ static const void* pick_fk64(bool adaptive, int fk, int ppt) {
 static const void* select_kernel64(const BorisArgs& a, bool queue) {
     const bool multi = a.alg == TP_ALG_MULTISTEP || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
-    const int fk = field_config_of(a.f);
-    const int ppt = a.ppt;
-    if (multi) return queue ? pick_fk64<true, true>(adaptive, fk, ppt) : pick_fk64<true, false>(adaptive, fk, ppt);
-    return queue ? pick_fk64<false, true>(adaptive, fk, ppt) : pick_fk64<false, false>(adaptive, fk, ppt);
+    if (multi) return queue ? pick_fk64<true, true>(adaptive, a) : pick_fk64<true, false>(adaptive, a);
+    return queue ? pick_fk64<false, true>(adaptive, a) : pick_fk64<false, false>(adaptive, a);
 }
 
 cudaError_t launch_boris_fp64(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s) {

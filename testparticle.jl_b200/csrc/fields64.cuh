@@ -6,6 +6,7 @@
 // +, -, *, /, sqrt and fma are involved.
 #pragma once
 
+#include "fdiv64.cuh"
 #include "grid_general.cuh"
 #include "ptrig.cuh"
 #include "tp_device.cuh"
@@ -335,8 +336,14 @@ __device__ __forceinline__ D3 boris_rot64(D3 v, D3 E, D3 B, double q2m, double d
 }
 
 // update_velocity_multistep, src/boris/multistep_boris.jl:65-142
-__device__ __forceinline__ D3 multistep_rot64(D3 v, D3 E, D3 B, double q2m, double dt, int N,
-                                              int n) {
+// split into the rotation, which depends on the fields and dt, and its
+// application to a velocity
+struct MultistepRot64 {
+    double c1, c2, c3, c6;
+    D3 t, e;
+};
+
+__device__ __forceinline__ MultistepRot64 multistep_rotation64(D3 E, D3 B, double q2m, double dt, int N, int n) {
     double factor = q2m * dt / (double)(2 * n);
     D3 t_n = factor * B;
     D3 e_n = factor * E;
@@ -377,16 +384,93 @@ __device__ __forceinline__ D3 multistep_rot64(D3 v, D3 E, D3 B, double q2m, doub
         c3 = 2.0 * s * s / t_n_mag2;
         c6 = (2.0 * nd - c2) / t_n_mag2;
     }
-    double v_dot_t = dot(v, t_n);
-    double e_dot_t = dot(e_n, t_n);
-    D3 v_cross_t = cross(v, t_n);
-    D3 e_cross_t = cross(e_n, t_n);
-    D3 out = c1 * v + c2 * v_cross_t;
-    out = out + (c3 * v_dot_t) * t_n;
-    out = out + c2 * e_n;
-    out = out + c3 * e_cross_t;
-    out = out + (c6 * e_dot_t) * t_n;
+    return {c1, c2, c3, c6, t_n, e_n};
+}
+
+__device__ __forceinline__ D3 multistep_rot64(D3 v, D3 E, D3 B, double q2m, double dt, int N,
+                                              int n) {
+    const MultistepRot64 m = multistep_rotation64(E, B, q2m, dt, N, n);
+    double v_dot_t = dot(v, m.t);
+    double e_dot_t = dot(m.e, m.t);
+    D3 v_cross_t = cross(v, m.t);
+    D3 e_cross_t = cross(m.e, m.t);
+    D3 out = m.c1 * v + m.c2 * v_cross_t;
+    out = out + (m.c3 * v_dot_t) * m.t;
+    out = out + m.c2 * m.e;
+    out = out + m.c3 * e_cross_t;
+    out = out + (m.c6 * e_dot_t) * m.t;
     return out;
+}
+
+// ---------------------------------------------------------------- E zero, B a dipole (FK_DIPOLE)
+// The arithmetic of analytic_eval64 / boris_rot64 / multistep_rot64 with the
+// shared reciprocals of fdiv64.cuh and without the terms of a zero E: 237
+// float64-pipe instructions per Multistep step instead of 358.  The float64
+// pipe (16 lanes per sub-partition) is what bounds these kernels.  They return
+// false, with nothing computed, where a denominator is outside the range of
+// fdiv64.cuh (the caller takes the general functions); NaN passes through.
+__device__ __forceinline__ bool dipole_fast64(const DevField& f, D3 r, D3& B) {
+    const D3 d = r - D3{f.c[0], f.c[1], f.c[2]};
+    const double d2 = abs2sum(d);
+    if (!in_range64(d2) && !isnan(d2)) return false;
+    const double y = rsqrt64(d2);
+    const double dm = sqrt64(d2, y);
+    const Rec64 q = rec64(dm, y);
+    const D3 rh{quot64(d.x, q), quot64(d.y, q), quot64(d.z, q)};
+    const double mr = dot(D3{f.m[0], f.m[1], f.m[2]}, rh);
+    const double d3 = (dm * dm) * dm;
+    const Rec64 q3 = rec64(d3, (y * y) * y);
+    const double s = 3.0 * mr;
+    B = {quot64(f.coef * (s * rh.x - f.m[0]), q3), quot64(f.coef * (s * rh.y - f.m[1]), q3),
+         quot64(f.coef * (s * rh.z - f.m[2]), q3)};
+    return true;
+}
+
+// boris_rot64 with E zero; qdt = q2m * 0.5 * dt
+__device__ __forceinline__ bool boris_fast64(D3 v, D3 B, double qdt, D3& out) {
+    const D3 t = qdt * B;
+    const double b = 1.0 + abs2sum(t);
+    if (!in_range64(b) && !isnan(b)) return false;
+    const Rec64 q = rec64(b, rcp64(b));
+    const D3 s{quot64(2.0 * t.x, q), quot64(2.0 * t.y, q), quot64(2.0 * t.z, q)};
+    const D3 vp = v + cross(v, t);
+    out = v + cross(vp, s);
+    return true;
+}
+
+// multistep_rot64 with E zero; factor = q2m * dt / (2n).  ORD: 2, 4 or 6
+template <int ORD>
+__device__ __forceinline__ bool multistep_fast64(D3 v, D3 B, double factor, int n, D3& out) {
+    D3 t = factor * B;
+    if (ORD != 2) {
+        const double m2 = abs2sum(t);
+        double f = 1.0 + third64(m2);
+        if (ORD == 6) f = f + fifteenth64(2.0 * m2 * m2);
+        t = f * t;
+    }
+    const double m2 = abs2sum(t);
+    const double nd = (double)n;
+    double c1, c2, c3;
+    if (m2 < 0x1.5798ee2308c3ap-27) {  // sqrt(m2) < 1e-4: the reference's Taylor branch
+        const double n1 = 2.0 * nd, n3 = 4.0 * nd * nd * nd;
+        c1 = fma(-(2.0 * nd * nd), m2, 1.0);
+        c2 = fma(-third64(n1 + n3), m2, n1);
+        c3 = fma(-third64(4.0 * nd * nd + 2.0 * nd * nd * nd * nd), m2, 2.0 * nd * nd);
+    } else {
+        if (!in_range64(m2) && !isnan(m2)) return false;
+        const double y = rsqrt64(m2);
+        const double m = sqrt64(m2, y);
+        const double a = patan01(m <= 1.0 ? m : 1.0 / m);
+        double s, c;
+        psincos<false>(nd * (m <= 1.0 ? a : 1.5707963267948966 - a), s, c);
+        c1 = fma(c, c, -(s * s));
+        c2 = quot64(2.0 * s * c, rec64(m, y));
+        c3 = quot64(2.0 * s * s, rec64(m2, y * y));
+    }
+    const double vt = c3 * dot(v, t);
+    const D3 x = cross(v, t);
+    out = (c1 * v + c2 * x) + vt * t;
+    return true;
 }
 
 template <bool MULTI>
@@ -402,8 +486,8 @@ __device__ __forceinline__ bool outside64(const DevTerm& T, D3 r, D3 v, double t
         if (isnan(r.x) || isnan(r.y) || isnan(r.z) || isnan(v.x) || isnan(v.y) || isnan(v.z))
             return true;
     if (f & TP_TERM_SHELL) {
-        double rr = sqrt((r.x * r.x + r.y * r.y) + r.z * r.z);
-        if (rr < T.rmin || rr > T.rmax) return true;
+        const double s = (r.x * r.x + r.y * r.y) + r.z * r.z;
+        if (s < T.smin || s > T.smax) return true;
     }
     if (f & TP_TERM_BOX) {
         if (r.x < T.lo[0] || r.x > T.hi[0]) return true;

@@ -68,8 +68,8 @@ __device__ __forceinline__ bool outside_gc(const DevTerm& T, const G4& u, double
         for (int k = 0; k < 4; ++k)
             if (isnan(u.y[k])) return true;
     if (f & TP_TERM_SHELL) {
-        double rr = sqrt((u.y[0] * u.y[0] + u.y[1] * u.y[1]) + u.y[2] * u.y[2]);
-        if (rr < T.rmin || rr > T.rmax) return true;
+        const double s = (u.y[0] * u.y[0] + u.y[1] * u.y[1]) + u.y[2] * u.y[2];
+        if (s < T.smin || s > T.smax) return true;
     }
     if (f & TP_TERM_BOX)
         for (int c = 0; c < 3; ++c)

@@ -18,6 +18,8 @@ namespace tpb {
 //   atan    for t in [0, 1]: up to two half-angle reductions tan(a/2) =
 //           t / (1 + sqrt(1 + t^2)) to t <= tan(pi/16), then the Taylor
 //           series to degree 29
+// WIDE = false: |x| < 2^31, so the quadrant fits an int (no 64-bit conversion)
+template <bool WIDE = true>
 __device__ __forceinline__ void psincos(double x, double& s, double& c) {
     const double P1 = 1.570796325802803, P2 = 9.920935791635221e-10, P3 = 5.170182981794105e-19;
     const double kf = rint(x * 0.6366197723675814);
@@ -46,7 +48,7 @@ __device__ __forceinline__ void psincos(double x, double& s, double& c) {
     pc = -1.0 / 24.0 + r2 * pc;
     pc = 0.5 + r2 * pc;
     const double cr = 1.0 - r2 * pc;
-    const int q = (int)((long long)kf & 3);
+    const int q = WIDE ? (int)((long long)kf & 3) : ((int)kf & 3);
     if (q == 0) {
         s = sr;
         c = cr;

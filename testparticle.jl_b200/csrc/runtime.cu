@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <string>
@@ -458,6 +459,24 @@ DevTerm dev_term(const tp_term_desc& t) {
         d.hi[k] = t.hi[k];
     }
     d.tmax = t.tmax;
+    // smallest s with sqrt(s) >= rmin and largest s with sqrt(s) <= rmax
+    const double big = std::numeric_limits<double>::infinity();
+    d.smin = t.rmin > 0.0 ? t.rmin * t.rmin : (t.rmin <= 0.0 ? 0.0 : t.rmin);
+    if (t.rmin > 0.0) {
+        while (d.smin > 0.0 && std::sqrt(std::nextafter(d.smin, 0.0)) >= t.rmin) d.smin = std::nextafter(d.smin, 0.0);
+        while (std::sqrt(d.smin) < t.rmin) d.smin = std::nextafter(d.smin, big);
+    }
+    d.smax = t.rmax >= 0.0 ? t.rmax * t.rmax : (t.rmax < 0.0 ? -1.0 : t.rmax);
+    if (t.rmax >= 0.0) {
+        while (std::sqrt(d.smax) > t.rmax) d.smax = std::nextafter(d.smax, 0.0);
+        while (d.smax < big && std::sqrt(std::nextafter(d.smax, big)) <= t.rmax) d.smax = std::nextafter(d.smax, big);
+    }
+    d.smin32 = t.rmin > 0.0 ? (float)(t.rmin * t.rmin) : -1.0f;
+    d.smax32 = t.rmax >= 0.0 ? (float)(t.rmax * t.rmax) : -1.0f;
+    for (int k = 0; k < 3; ++k) {
+        d.lo32[k] = (float)t.lo[k];
+        d.hi32[k] = (float)t.hi[k];
+    }
     return d;
 }
 

@@ -105,6 +105,12 @@ struct DevTerm {
     double rmin, rmax;
     double lo[3], hi[3];
     double tmax;
+    // the shell test on squared radii: sqrt(s) < rmin exactly when s < smin,
+    // sqrt(s) > rmax exactly when s > smax (the rounded root is monotone in s),
+    // so no kernel takes a square root per step for it
+    double smin, smax;
+    // the float forms the FP32C kernels test against (squared shell radii, box)
+    float smin32, smax32, lo32[3], hi32[3];
 };
 
 // Field configurations a kernel is specialised for (keeps register use down):
@@ -113,7 +119,10 @@ struct DevTerm {
 //   FK_GENERIC   anything else (separate grids, grid + analytic)
 //   FK_GENGRID   at least one grid off the trilinear uniform Cartesian path
 //                (order 0 / 3, rectilinear, spherical, 1-D / 2-D)
-enum { FK_ANALYTIC = 0, FK_EBGRID = 1, FK_GENERIC = 2, FK_GENGRID = 3 };
+// and, inside FK_ANALYTIC, the two configurations with kernels of their own
+//   FK_DIPOLE    E zero, B a dipole
+//   FK_UNIFORM   E and B each zero or uniform
+enum { FK_ANALYTIC = 0, FK_EBGRID = 1, FK_GENERIC = 2, FK_GENGRID = 3, FK_DIPOLE = 4, FK_UNIFORM = 5 };
 
 __host__ __device__ __forceinline__ int field_config_of(const DevFields& f) {
     if ((f.E.kind == TP_FIELD_GRID && f.E.general) || (f.B.kind == TP_FIELD_GRID && f.B.general) ||
@@ -123,6 +132,16 @@ __host__ __device__ __forceinline__ int field_config_of(const DevFields& f) {
     if (f.eb && !f.eb_f64) return FK_EBGRID;  // float interleaved table
     if (f.E.kind != TP_FIELD_GRID && f.B.kind != TP_FIELD_GRID) return FK_ANALYTIC;
     return FK_GENERIC;
+}
+
+// the configuration a full-orbit kernel is compiled for
+__host__ __device__ __forceinline__ int kernel_config_of(const DevFields& f) {
+    const int fk = field_config_of(f);
+    if (fk != FK_ANALYTIC) return fk;
+    if (f.E.kind == TP_FIELD_ZERO && f.B.kind == TP_FIELD_DIPOLE) return FK_DIPOLE;
+    const bool ue = f.E.kind == TP_FIELD_ZERO || f.E.kind == TP_FIELD_UNIFORM;
+    const bool ub = f.B.kind == TP_FIELD_ZERO || f.B.kind == TP_FIELD_UNIFORM;
+    return ue && ub ? FK_UNIFORM : FK_ANALYTIC;
 }
 
 // ------------------------------------------------------------------ launch
