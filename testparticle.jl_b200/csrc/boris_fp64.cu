@@ -428,11 +428,7 @@ static const void* kernel_ptr64(bool adaptive, int ppt) {
 
 template <bool MULTI, bool QUEUE>
 static const void* pick_fk64(bool adaptive, const BorisArgs& a) {
-    const int fk = kernel_config_of(a.f);
-    if (fk == FK_DIPOLE || fk == FK_UNIFORM) {
-        if (!adaptive && a.ppt != 2) return seg_kernel64(a, QUEUE);
-        return kernel_ptr64<MULTI, QUEUE, FK_ANALYTIC>(adaptive, a.ppt);
-    }
+    const int fk = field_config_of(a.f);
     if (fk == FK_ANALYTIC) return kernel_ptr64<MULTI, QUEUE, FK_ANALYTIC>(adaptive, a.ppt);
     if (fk == FK_EBGRID) return kernel_ptr64<MULTI, QUEUE, FK_EBGRID>(adaptive, 1);
     if (fk == FK_GENGRID) return kernel_ptr64<MULTI, QUEUE, FK_GENGRID>(adaptive, 1);
@@ -440,6 +436,7 @@ static const void* pick_fk64(bool adaptive, const BorisArgs& a) {
 }
 
 static const void* select_kernel64(const BorisArgs& a, bool queue) {
+    if (seg_config(a)) return seg_kernel64(a, queue);
     const bool multi = a.alg == TP_ALG_MULTISTEP || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     if (multi) return queue ? pick_fk64<true, true>(adaptive, a) : pick_fk64<true, false>(adaptive, a);

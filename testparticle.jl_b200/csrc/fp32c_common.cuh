@@ -525,6 +525,19 @@ __device__ __forceinline__ D3 cpos_d3(const CPos& p) {
             (double)p.hi[2] + (double)p.lo[2]};
 }
 
+__device__ __forceinline__ D3 dipole_mixed(const DevField& f, const CPos& p) {
+    // B = coef (3 (m.d) d / r^5 - m / r^3), 1/r = y (1.5 - r^2 y^2 / 2)
+    // from the float estimate y (relative error ~1e-13 after the step)
+    const D3 d = cpos_d3(p) - D3{f.c[0], f.c[1], f.c[2]};
+    const double r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+    double y = (double)rsqrtf((float)r2);
+    y = y * fma(-0.5 * r2, y * y, 1.5);
+    const double ir2 = y * y;
+    const double k3 = f.coef * (ir2 * y);
+    const double k5 = 3.0 * (k3 * ir2) * (f.m[0] * d.x + f.m[1] * d.y + f.m[2] * d.z);
+    return {k5 * d.x - k3 * f.m[0], k5 * d.y - k3 * f.m[1], k5 * d.z - k3 * f.m[2]};
+}
+
 // analytic field in float64 at a compensated position
 __device__ __forceinline__ D3 analytic_eval_mixed(const DevField& f, const CPos& p, double t) {
     switch (f.kind) {
@@ -536,18 +549,8 @@ __device__ __forceinline__ D3 analytic_eval_mixed(const DevField& f, const CPos&
                     f.v[1] + f.J[3] * r.x + f.J[4] * r.y + f.J[5] * r.z + f.rate[1] * t,
                     f.v[2] + f.J[6] * r.x + f.J[7] * r.y + f.J[8] * r.z + f.rate[2] * t};
         }
-        case TP_FIELD_DIPOLE: {
-            // B = coef (3 (m.d) d / r^5 - m / r^3), 1/r = y (1.5 - r^2 y^2 / 2)
-            // from the float estimate y (relative error ~1e-13 after the step)
-            const D3 d = cpos_d3(p) - D3{f.c[0], f.c[1], f.c[2]};
-            const double r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-            double y = (double)rsqrtf((float)r2);
-            y = y * fma(-0.5 * r2, y * y, 1.5);
-            const double ir2 = y * y;
-            const double k3 = f.coef * (ir2 * y);
-            const double k5 = 3.0 * (k3 * ir2) * (f.m[0] * d.x + f.m[1] * d.y + f.m[2] * d.z);
-            return {k5 * d.x - k3 * f.m[0], k5 * d.y - k3 * f.m[1], k5 * d.z - k3 * f.m[2]};
-        }
+        case TP_FIELD_DIPOLE:
+            return dipole_mixed(f, p);
         default:
             return {0.0, 0.0, 0.0};
     }
@@ -557,7 +560,13 @@ __device__ __forceinline__ D3 analytic_eval_mixed(const DevField& f, const CPos&
 // which is its n = 1, N = 2 case (c1 + 1 = c2 = c3 = c6 = 2 / (1 + |t|^2)) --
 // with fac = q2m dt / (2n): float rotation factors from the float copy of
 // the axis, refined as above, applied in float64.
-__device__ __forceinline__ D3 rot_mixed(D3 v, D3 E, D3 B, double fac, int N, int n, bool hasE) {
+// The rotation (fields and fac only) and its application to a velocity.
+struct RotMixed {
+    D3 t, e;
+    double C1, C2, C3, c6;
+};
+
+__device__ __forceinline__ RotMixed rotation_mixed(D3 E, D3 B, double fac, int N, int n, bool hasE) {
     D3 t = fac * B;
     D3 e = hasE ? fac * E : D3{0.0, 0.0, 0.0};
     double sd = dot(t, t);
@@ -577,8 +586,8 @@ __device__ __forceinline__ D3 rot_mixed(D3 v, D3 E, D3 B, double fac, int N, int
         sd = (fd * fd) * sd;
         s = (float)sd;
     }
-    float zr = 1.0f, q = 0.0f, A = 1.0f, R = 0.0f;
-    for (int k = 0; k < n; ++k) {
+    float zr = 1.0f, q = 1.0f, A = 1.0f + s, R = 1.0f;  // after the first of the n >= 1 substeps
+    for (int k = 1; k < n; ++k) {
         R = R + (float)(k + 1) * A + 2.0f * q * q + zr * q;
         float nzr = zr - s * q;
         q = zr + q;
@@ -598,13 +607,18 @@ __device__ __forceinline__ D3 rot_mixed(D3 v, D3 E, D3 B, double fac, int N, int
     C2 = C2 - hg * C2;
     const float rs = s > 0.0f ? __fdividef(1.0f, s) : 0.0f;
     C3 = C3 - fma(C3, sd, C1) * (double)rs;
-    const D3 vxt = cross(v, t);
-    D3 dv = C1 * v + C2 * vxt + (C3 * dot(v, t)) * t;
-    if (hasE) {
-        const double c6 = (2.0 * R) * invA;
-        dv = dv + C2 * e + C3 * cross(e, t) + (c6 * dot(e, t)) * t;
-    }
+    return {t, e, C1, C2, C3, hasE ? (2.0 * R) * invA : 0.0};
+}
+
+__device__ __forceinline__ D3 rotate_mixed(D3 v, const RotMixed& m, bool hasE) {
+    const D3 vxt = cross(v, m.t);
+    D3 dv = m.C1 * v + m.C2 * vxt + (m.C3 * dot(v, m.t)) * m.t;
+    if (hasE) dv = dv + m.C2 * m.e + m.C3 * cross(m.e, m.t) + (m.c6 * dot(m.e, m.t)) * m.t;
     return v + dv;
+}
+
+__device__ __forceinline__ D3 rot_mixed(D3 v, D3 E, D3 B, double fac, int N, int n, bool hasE) {
+    return rotate_mixed(v, rotation_mixed(E, B, fac, N, n, hasE), hasE);
 }
 
 // velocity update of length dt, fields (E, B) in float64

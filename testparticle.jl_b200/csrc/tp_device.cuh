@@ -181,6 +181,14 @@ struct BorisArgs {
     int64_t done_chunk;
 };
 
+// the run takes the kernels of seg_common.cuh: one particle per thread, a
+// dipole or uniform fields with fixed steps, or a dipole with AdaptiveBoris
+__host__ __forceinline__ bool seg_config(const BorisArgs& a) {
+    const int fk = kernel_config_of(a.f);
+    if (a.alg == TP_ALG_ADAPTIVE) return fk == FK_DIPOLE;
+    return (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP) && (fk == FK_DIPOLE || fk == FK_UNIFORM) && a.ppt != 2;
+}
+
 // particle i's outputs are final: publish them, then count the particle
 __device__ __forceinline__ void particle_done(const BorisArgs& a, int64_t i) {
     if (a.done) {

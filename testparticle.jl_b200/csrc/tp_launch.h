@@ -159,8 +159,9 @@ cudaError_t launch_table_sum(const float4* tab, int64_t nodes, int stride, int o
 cudaError_t launch_table_unpack(const float4* tab, int64_t nodes, int stride, int off, int G, double* out,
                                 cudaStream_t s);
 
-// the fixed-step kernel of a dipole or uniform-field run (boris_seg64.cu)
+// the kernel of a run that seg_config() accepts (boris_seg64.cu, boris_seg32.cu)
 const void* seg_kernel64(const BorisArgs& a, bool queue);
+const void* seg_kernel32(const BorisArgs& a, bool queue);
 cudaError_t launch_boris_fp64(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s);
 cudaError_t launch_boris_fp32c(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s);
 // the FP32C run takes the warp-cooperative cubic-grid kernel (static schedule only)
