@@ -129,7 +129,7 @@ __device__ __forceinline__ F3 vminus(F3 v, F3 E, float h) {
 // for any E), so records of the fused backward keep vm instead of both.
 __device__ __forceinline__ UAdj u_adjoint_vm(F3 vm, F3 B, float h, F3 lo) {
     F3 t = h * B;
-    float sc = 2.0f * __frcp_rn(1.0f + dot(t, t));
+    float sc = 2.0f * __frcp_rn(1.0f + dot_fma<2>(t, t));
     F3 vp = vm + cross(vm, t);
     F3 s = sc * t;
     F3 ls = cross(lo, vp);
@@ -161,6 +161,13 @@ __device__ __forceinline__ void tri_nodes(const DevField& g, const AxF& ax, cons
     nd[5] = ax.i1 + j0 + k1;
     nd[6] = ax.i0 + j1 + k1;
     nd[7] = ax.i1 + j1 + k1;
+}
+
+// the same in the interleaved E/B table
+__device__ __forceinline__ void tri_nodes_eb(const DevField& g, const AxF& ax, const AxF& ay, const AxF& az, int* nd) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        nd[c] = eb_node(g, (c & 1) ? ax.i1 : ax.i0, (c & 2) ? ay.i1 : ay.i0, (c & 4) ? az.i1 : az.i0);
 }
 
 __device__ __forceinline__ void tri_weights(const AxF& ax, const AxF& ay, const AxF& az, float* w) {
@@ -344,7 +351,7 @@ __device__ __forceinline__ F3 adj_step_eb(const AdjArgs& A, const CPos& p, F3 v,
         return nanf3_();
     }
     int nd[8];
-    tri_nodes(F.B, ax, ay, az, nd);
+    tri_nodes_eb(F.B, ax, ay, az, nd);
     F3 E, B, Ex, Ey, Ez, Bx, By, Bz;
     {
         const float4* T = F.eb32;
@@ -637,7 +644,7 @@ __device__ __forceinline__ void record_step_eb(const AdjArgs& A, const CPos& p, 
         return;
     }
     int nd[8];
-    tri_nodes(F.B, ax, ay, az, nd);
+    tri_nodes_eb(F.B, ax, ay, az, nd);
     float4 e[8], b[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) ldg_node8(F.eb32 + 2 * (int64_t)nd[c], e[c], b[c]);
@@ -743,7 +750,7 @@ __device__ __forceinline__ void scatter_warp_eb(const AdjArgs& A, float* stage, 
         }
         int nd[8];
         float w[8];
-        tri_nodes(g, ax, ay, az, nd);
+        tri_nodes_eb(g, ax, ay, az, nd);
         tri_weights(ax, ay, az, w);
         float4* me = reinterpret_cast<float4*>(stage + lane * kStage);
         me[0] = make_float4(__int_as_float(nd[0]), __int_as_float(nd[1]), __int_as_float(nd[2]), __int_as_float(nd[3]));
@@ -943,7 +950,7 @@ __device__ __forceinline__ void record_step_f(const DevFields& F, const CPos& p,
         return;
     }
     int nd[8];
-    tri_nodes(F.B, ax, ay, az, nd);
+    tri_nodes_eb(F.B, ax, ay, az, nd);
     float4 e[8], b[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) ldg_node8(F.eb32 + 2 * (int64_t)nd[c], e[c], b[c]);
@@ -1045,7 +1052,7 @@ __global__ void __launch_bounds__(128, 3) k_adj_fused_eb(AdjArgs A) {
                 for (int j = 0; j < m; ++j) {
                     F3 E, B;
                     record_step_f(a.f, p, v.h, h, mine + j * kRecF2 * stride, stride, E, B);
-                    v = vel32h<false>(v, E, B, a, h);
+                    v = vel32h<false, 1>(v, E, B, a, h);
                     cpos_push_cv(a, p, v, dth, dtl);
                 }
                 if (s == A.S - 1) {  // the final save's update, at (x_N, v_{N-1/2})
@@ -1121,6 +1128,29 @@ __global__ void k_table_unpack(const float4* tab, int64_t nodes, int stride, int
     out[3 * k + 2] = ldexp((double)q.z, G);
 }
 
+// The E (off 0) or B (off 1) half of the interleaved node-gradient table, z
+// fastest, into the user layout, x fastest: tiles of 32 x 32 nodes in (x, z)
+// turned in shared memory, so that reads and writes are both contiguous.
+__global__ void __launch_bounds__(256) k_eb_unpack(const float4* tab, int nx, int ny, int nz, int off, int G, double* out) {
+    __shared__ float4 tile[32][33];
+    const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32, lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    for (int y = blockIdx.z; y < ny; y += gridDim.z) {
+        for (int r = row; r < 32; r += 8)
+            if (x0 + r < nx && z0 + lane < nz)
+                tile[r][lane] = tab[2 * (z0 + lane + (int64_t)nz * (y + (int64_t)ny * (x0 + r))) + off];
+        __syncthreads();
+        for (int r = row; r < 32; r += 8)
+            if (x0 + lane < nx && z0 + r < nz) {
+                const float4 q = tile[lane][r];
+                double* o = out + 3 * (x0 + lane + (int64_t)nx * (y + (int64_t)ny * (z0 + r)));
+                o[0] = ldexp((double)q.x, G);
+                o[1] = ldexp((double)q.y, G);
+                o[2] = ldexp((double)q.z, G);
+            }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------------- launchers
 int adjoint_field_config(const DevFields& f) {
     if (f.eb32) return FK_EBGRID;
@@ -1194,6 +1224,12 @@ cudaError_t launch_table_unpack(const float4* tab, int64_t nodes, int stride, in
     if (nodes <= 0) return cudaSuccess;
     const int block = 256;
     k_table_unpack<<<(unsigned)((nodes + block - 1) / block), block, 0, s>>>(tab, nodes, stride, off, G, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_eb_unpack(const float4* tab, const int32_t n[3], int off, int G, double* out, cudaStream_t s) {
+    const dim3 grid((n[0] + 31) / 32, (n[2] + 31) / 32, n[1] < 65535 ? n[1] : 65535);
+    k_eb_unpack<<<grid, 256, 0, s>>>(tab, n[0], n[1], n[2], off, G, out);
     return cudaGetLastError();
 }
 

@@ -75,6 +75,25 @@ struct Saver32 {
     }
 };
 
+// save slot 0: u0 itself, and the fields as the push sees them
+template <int FK>
+__device__ __forceinline__ void save_first32(const BorisArgs& a, int64_t i, const CPos& p) {
+    if (a.nslots < 1) {
+        set_status(a.status, TP_E_OVERFLOW);
+        return;
+    }
+    a.t_out[i] = a.t0;
+    const double* u0 = a.u0 + 6 * i;
+    double* u = a.u_out + i;
+    for (int c = 0; c < 6; ++c) u[c * a.n] = u0[c];
+    if (a.save_fields) {
+        typename Vel32<FK>::Fv E, B;
+        Vel32<FK>::fields(a.f, p, a.t0, E, B);
+        u[6 * a.n] = E.x; u[7 * a.n] = E.y; u[8 * a.n] = E.z;
+        u[9 * a.n] = B.x; u[10 * a.n] = B.y; u[11 * a.n] = B.z;
+    }
+}
+
 }  // namespace
 
 }  // namespace tpb

@@ -821,6 +821,7 @@ static const void* select_kernel32(const BorisArgs& a, bool queue) {
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     if (cubic_coop_kernel(a)) return multi ? (const void*)k_cubic32c<true> : (const void*)k_cubic32c<false>;
     if (seg_config(a)) return seg_kernel32(a, queue);
+    if (field_config_of(a.f) == FK_EBGRID && !adaptive) return grid_kernel32(a, queue);
     const int fk = field_config_of(a.f);
     const int ppt = a.ppt;
     if (multi) return queue ? pick_fk32<true, true>(adaptive, fk, ppt) : pick_fk32<true, false>(adaptive, fk, ppt);

@@ -31,23 +31,16 @@ struct Push32 {
         cpos_init(a, p, u0);
         v = {u0[3], u0[4], u0[5]};
     }
-    // u0 itself, and the fields as the push sees them
     static __device__ __forceinline__ void save_first(const BorisArgs& a, const Saver&, int64_t i, const CPos& p, D3) {
-        if (a.nslots < 1) {
-            set_status(a.status, TP_E_OVERFLOW);
-            return;
-        }
-        a.t_out[i] = a.t0;
-        const double* u0 = a.u0 + 6 * i;
-        double* u = a.u_out + i;
-        for (int c = 0; c < 6; ++c) u[c * a.n] = u0[c];
-        if (a.save_fields) {
-            const D3 E = analytic_eval_mixed(a.f.E, p, a.t0), B = analytic_eval_mixed(a.f.B, p, a.t0);
-            u[6 * a.n] = E.x; u[7 * a.n] = E.y; u[8 * a.n] = E.z;
-            u[9 * a.n] = B.x; u[10 * a.n] = B.y; u[11 * a.n] = B.z;
-        }
+        save_first32<FK_ANALYTIC>(a, i, p);
     }
     static __device__ __forceinline__ D3 general(const BorisArgs& a, const CPos& p, D3 v, double dt) {
+        return kick_general32<MULTI>(a, p, v, dt);
+    }
+    struct F {};
+    static constexpr bool kWarp = false;
+    static __device__ __forceinline__ F fields(const BorisArgs&, const CPos&) { return {}; }
+    static __device__ __forceinline__ D3 update(const BorisArgs& a, const CPos& p, D3 v, F, double dt) {
         return kick_general32<MULTI>(a, p, v, dt);
     }
     static __device__ __forceinline__ CPos advance(const BorisArgs& a, CPos p, D3 v, double dt) {
@@ -70,7 +63,7 @@ struct DipolePush32 : Push32<MULTI> {
     __device__ __forceinline__ void start(const BorisArgs& a, double dt) {
         h = MULTI ? a.q2m * dt / (double)(2 * a.nsub) : a.q2m * 0.5 * dt;
     }
-    __device__ __forceinline__ bool kick(const BorisArgs& a, const CPos& p, D3 v, D3& out) const {
+    __device__ __forceinline__ bool kick(const BorisArgs& a, const CPos& p, D3 v, typename Push32<MULTI>::F, D3& out) const {
         out = rot_mixed(v, D3{0.0, 0.0, 0.0}, dipole_mixed(a.f.B, p), h, ORD, MULTI ? a.nsub : 1, false);
         return true;
     }
@@ -108,7 +101,7 @@ struct UniformPush32 : Push32<MULTI> {
         m = MULTI ? rotation_mixed(E, B, a.q2m * dt / (double)(2 * a.nsub), a.order, a.nsub, hasE)
                   : rotation_mixed(E, B, a.q2m * 0.5 * dt, 2, 1, hasE);
     }
-    __device__ __forceinline__ bool kick(const BorisArgs& a, const CPos&, D3 v, D3& out) const {
+    __device__ __forceinline__ bool kick(const BorisArgs& a, const CPos&, D3 v, typename Push32<MULTI>::F, D3& out) const {
         out = rotate_mixed(v, m, a.f.E.kind != TP_FIELD_ZERO);
         return true;
     }

@@ -38,6 +38,12 @@ struct Push64 {
     static __device__ __forceinline__ D3 general(const BorisArgs& a, D3 r, D3 v, double dt) {
         return kick_general64<MULTI>(a, r, v, dt);
     }
+    struct F {};
+    static constexpr bool kWarp = false;
+    static __device__ __forceinline__ F fields(const BorisArgs&, D3) { return {}; }
+    static __device__ __forceinline__ D3 update(const BorisArgs& a, D3 r, D3 v, F, double dt) {
+        return kick_general64<MULTI>(a, r, v, dt);
+    }
     static __device__ __forceinline__ D3 advance(const BorisArgs&, D3 r, D3 v, double dt) { return r + v * dt; }
     static __device__ __forceinline__ bool outside(const BorisArgs& a, D3 r, D3 v, double t) {
         return outside64(a.term, r, v, t);
@@ -55,7 +61,7 @@ struct DipolePush64 : Push64<MULTI> {
     __device__ __forceinline__ void start(const BorisArgs& a, double dt) {
         h = MULTI ? a.q2m * dt / (double)(2 * a.nsub) : a.q2m * 0.5 * dt;
     }
-    __device__ __forceinline__ bool kick(const BorisArgs& a, D3 r, D3 v, D3& out) const {
+    __device__ __forceinline__ bool kick(const BorisArgs& a, D3 r, D3 v, typename Push64<MULTI>::F, D3& out) const {
         D3 B;
         return dipole_fast64(a.f.B, r, B) &&
                (MULTI ? multistep_fast64<ORD>(v, B, h, a.nsub, out) : boris_fast64(v, B, h, out));
@@ -97,7 +103,7 @@ struct UniformPush64<false> : Push64<false> {
         s = (2.0 * t) / (1.0 + abs2sum(t));
         he = h * analytic_eval64(a.f.E, z, 0.0);
     }
-    __device__ __forceinline__ bool kick(const BorisArgs&, D3, D3 v, D3& out) const {
+    __device__ __forceinline__ bool kick(const BorisArgs&, D3, D3 v, F, D3& out) const {
         const D3 vm = v + he;
         const D3 vp = vm + cross(vm, t);
         out = (vm + cross(vp, s)) + he;
@@ -118,7 +124,7 @@ struct UniformPush64<true> : Push64<true> {
         e2 = m.c3 * cross(m.e, m.t);
         e3 = (m.c6 * dot(m.e, m.t)) * m.t;
     }
-    __device__ __forceinline__ bool kick(const BorisArgs&, D3, D3 v, D3& out) const {
+    __device__ __forceinline__ bool kick(const BorisArgs&, D3, D3 v, F, D3& out) const {
         out = m.c1 * v + m.c2 * cross(v, m.t);
         out = out + (m.c3 * dot(v, m.t)) * m.t;
         out = ((out + e1) + e2) + e3;

@@ -79,7 +79,7 @@ __device__ __forceinline__ D3 load_node(const void* tab, bool f64, int64_t idx) 
 }
 
 // Trilinear interpolation from precomputed axes; `stride`/`off` select a
-// field inside an interleaved table (stride 2: E at off 0, B at off 1).
+// field inside an interleaved table.
 __device__ __forceinline__ D3 tri64(const DevField& g, const void* tab, bool f64, int stride,
                                     int off, const Ax& ax, const Ax& ay, const Ax& az) {
     const int64_t nx = g.n[0], nxy = (int64_t)g.n[0] * g.n[1];
@@ -232,25 +232,6 @@ __device__ __forceinline__ D3 field_eval64(const DevField& f, D3 r, double t) {
     return analytic_eval64(f, r, t);
 }
 
-// E and B at one point (one gather pass when the two grids are interleaved).
-__device__ __forceinline__ void eval_EB64(const DevFields& F, D3 r, double t, D3& E, D3& B) {
-    if (F.eb) {
-        // both grids on one geometry: one axis computation, one gather pass
-        Ax ax, ay, az;
-        if (!grid_axes64(F.B, r, ax, ay, az)) {
-            E = nan3();
-            B = E;
-            return;
-        }
-        bool f64 = F.eb_f64 != 0;
-        E = tri64(F.B, F.eb, f64, 2, 0, ax, ay, az);
-        B = tri64(F.B, F.eb, f64, 2, 1, ax, ay, az);
-        return;
-    }
-    E = field_eval64(F.E, r, t);
-    B = field_eval64(F.B, r, t);
-}
-
 // One 32-byte node record (E xyz0, B xyz0) of the float interleaved table in
 // a single 256-bit read-only load (sm_100 ld.global.nc.v8).
 __device__ __forceinline__ void ldg_node8_64(const float4* p, float4& e, float4& b) {
@@ -269,18 +250,18 @@ __device__ __forceinline__ void eb_eval64_f32(const DevFields& F, D3 r, D3& E, D
         return;
     }
     const float4* T = F.eb32;
-    const int64_t nx = F.B.n[0], nxy = (int64_t)F.B.n[0] * F.B.n[1];
-    int64_t j0 = ay.i0 * nx, j1 = ay.i1 * nx, k0 = az.i0 * nxy, k1 = az.i1 * nxy;
     float4 e000, b000, e100, b100, e010, b010, e110, b110;
     float4 e001, b001, e101, b101, e011, b011, e111, b111;
-    ldg_node8_64(T + 2 * (ax.i0 + j0 + k0), e000, b000);
-    ldg_node8_64(T + 2 * (ax.i1 + j0 + k0), e100, b100);
-    ldg_node8_64(T + 2 * (ax.i0 + j1 + k0), e010, b010);
-    ldg_node8_64(T + 2 * (ax.i1 + j1 + k0), e110, b110);
-    ldg_node8_64(T + 2 * (ax.i0 + j0 + k1), e001, b001);
-    ldg_node8_64(T + 2 * (ax.i1 + j0 + k1), e101, b101);
-    ldg_node8_64(T + 2 * (ax.i0 + j1 + k1), e011, b011);
-    ldg_node8_64(T + 2 * (ax.i1 + j1 + k1), e111, b111);
+#define TPB_CORNER(X, Y, Z) ldg_node8_64(T + 2 * (int64_t)eb_node(F.B, ax.i##X, ay.i##Y, az.i##Z), e##X##Y##Z, b##X##Y##Z);
+    TPB_CORNER(0, 0, 0)
+    TPB_CORNER(1, 0, 0)
+    TPB_CORNER(0, 1, 0)
+    TPB_CORNER(1, 1, 0)
+    TPB_CORNER(0, 0, 1)
+    TPB_CORNER(1, 0, 1)
+    TPB_CORNER(0, 1, 1)
+    TPB_CORNER(1, 1, 1)
+#undef TPB_CORNER
 #define TPB_TRI64F(dst, q, c)                                                                  \
     {                                                                                          \
         double c00 = lerp64((double)(q##000).c, (double)(q##100).c, ax.f);                         \

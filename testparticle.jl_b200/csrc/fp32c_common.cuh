@@ -69,13 +69,11 @@ __device__ __forceinline__ void cpos_push(const BorisArgs& a, CPos& p, F3 v, flo
     for (int c = 0; c < 3; ++c) {
         cadd(p.hi[c], p.lo[c], d[c]);
         if (WRAP && a.wrap[c]) {
-            float x0 = (float)a.wrap0[c];
-            float L = (float)a.wrapL[c];
-            if (p.hi[c] >= x0 + L) {
-                cadd(p.hi[c], p.lo[c], -L);
+            if (p.hi[c] >= a.wrap1_32[c]) {
+                cadd(p.hi[c], p.lo[c], -a.wrapL32[c]);
                 p.w[c] += 1;
-            } else if (p.hi[c] < x0) {
-                cadd(p.hi[c], p.lo[c], L);
+            } else if (p.hi[c] < a.wrap0_32[c]) {
+                cadd(p.hi[c], p.lo[c], a.wrapL32[c]);
                 p.w[c] -= 1;
             }
         }
@@ -156,10 +154,41 @@ __device__ __forceinline__ bool axis32(const DevField& g, int a, float hi, float
         f += (float)(i - (na - 2));
         i = na - 2;
     }
+    i = max(i, 0);  // a clamped position of -inf
     o.i0 = i;
     o.i1 = i + 1;
     o.f = f;
     return true;
+}
+
+// axis32 on a periodic axis (o.ds aside).  Positions are kept in the box or near
+// it, so the index is in range but for rounding at the edges: one test covers
+// that, positions left unwrapped and NaN; and next to the nearest node only a
+// negative fraction needs a correction.
+__device__ __forceinline__ void axis32_periodic(const DevField& g, int a, float hi, float lo, AxF& o) {
+    const float kMagic = 12582912.0f;  // 1.5 * 2^23
+    const float d = hi - g.x0f[a];
+    const float u = d * g.idxf[a];
+    if (!(fabsf(u) < 4194304.0f)) {
+        axis32(g, a, hi, lo, o);
+        return;
+    }
+    const float tr = __fadd_rn(u, kMagic);
+    int i = __float_as_int(tr) - __float_as_int(kMagic);
+    const float rem = fmaf(-(tr - kMagic), g.dxf[a], d) + lo;
+    float f = rem * g.idxf[a];
+    if (f < 0.0f) {
+        i -= 1;
+        f += 1.0f;
+    }
+    const int na = g.n[a];
+    if ((unsigned)i >= (unsigned)na) {
+        i %= na;
+        if (i < 0) i += na;
+    }
+    o.i0 = i;
+    o.i1 = (i + 1 == na) ? 0 : i + 1;
+    o.f = f;
 }
 
 __device__ __forceinline__ float lerp32(float a, float b, float f) { return fmaf(f, b - a, a); }
@@ -268,24 +297,20 @@ __device__ __forceinline__ void eval_EB32(const DevFields& F, const CPos& p, dou
             return;
         }
         const float4* T = F.eb32;
-        const int nx = F.B.n[0], nxy = F.B.n[0] * F.B.n[1];
-        int j0 = ay.i0 * nx, j1 = ay.i1 * nx, k0 = az.i0 * nxy, k1 = az.i1 * nxy;
-        int n000 = 2 * (ax.i0 + j0 + k0), n100 = 2 * (ax.i1 + j0 + k0);
-        int n010 = 2 * (ax.i0 + j1 + k0), n110 = 2 * (ax.i1 + j1 + k0);
-        int n001 = 2 * (ax.i0 + j0 + k1), n101 = 2 * (ax.i1 + j0 + k1);
-        int n011 = 2 * (ax.i0 + j1 + k1), n111 = 2 * (ax.i1 + j1 + k1);
         // 8 corners, each one aligned 32-byte sector (E xyz0, B xyz0) read by
         // one 256-bit load; all issued before any use
         float4 e000, b000, e100, b100, e010, b010, e110, b110;
         float4 e001, b001, e101, b101, e011, b011, e111, b111;
-        ldg_node8(T + n000, e000, b000);
-        ldg_node8(T + n100, e100, b100);
-        ldg_node8(T + n010, e010, b010);
-        ldg_node8(T + n110, e110, b110);
-        ldg_node8(T + n001, e001, b001);
-        ldg_node8(T + n101, e101, b101);
-        ldg_node8(T + n011, e011, b011);
-        ldg_node8(T + n111, e111, b111);
+#define TPB_CORNER(X, Y, Z) ldg_node8(T + 2 * (int64_t)eb_node(F.B, ax.i##X, ay.i##Y, az.i##Z), e##X##Y##Z, b##X##Y##Z);
+        TPB_CORNER(0, 0, 0)
+        TPB_CORNER(1, 0, 0)
+        TPB_CORNER(0, 1, 0)
+        TPB_CORNER(1, 1, 0)
+        TPB_CORNER(0, 0, 1)
+        TPB_CORNER(1, 0, 1)
+        TPB_CORNER(0, 1, 1)
+        TPB_CORNER(1, 1, 1)
+#undef TPB_CORNER
         E = tri3(xyz(e000), xyz(e100), xyz(e010), xyz(e110), xyz(e001), xyz(e101), xyz(e011),
                  xyz(e111), ax, ay, az);
         B = tri3(xyz(b000), xyz(b100), xyz(b010), xyz(b110), xyz(b001), xyz(b101), xyz(b011),
@@ -422,11 +447,22 @@ __device__ __forceinline__ CV cv_from(const double* u) {
     return v;
 }
 
+// |t|^2 of a velocity update.  ORD 0 leaves the contraction to the compiler, which
+// chooses per call site; 1 and 2 spell out the two forms it takes, for kernels
+// whose results have to round like another kernel's.
+template <int ORD>
+__device__ __forceinline__ float dot_fma(F3 a, F3 b) {
+    if (ORD == 1) return fmaf(a.z, b.z, fmaf(a.y, b.y, __fmul_rn(a.x, b.x)));
+    if (ORD == 2) return fmaf(a.z, b.z, fmaf(a.x, b.x, __fmul_rn(a.y, b.y)));
+    return dot(a, b);
+}
+
 // Boris (boris.jl:19-31): dv = 2 h E + (v- + v- x t) x s,  h = q2m*dt/2,
 // s = 2 t / (1 + |t|^2) with a correctly rounded reciprocal
+template <int ORD = 0>
 __device__ __forceinline__ F3 boris_delta32(F3 v, F3 E, F3 B, float h) {
     F3 t = h * B;
-    float sc = 2.0f * __frcp_rn(1.0f + dot(t, t));
+    float sc = 2.0f * __frcp_rn(1.0f + dot_fma<ORD>(t, t));
     F3 he = h * E;
     F3 vm = v + he;
     F3 vp = vm + cross(vm, t);
@@ -439,10 +475,11 @@ __device__ __forceinline__ F3 boris_delta32(F3 v, F3 E, F3 B, float h) {
 //   dv = (c1 - 1) v + c2 v x t + c3 (v.t) t + c2 e + c3 e x t + c6 (e.t) t
 // with c1 - 1 = -2 s q^2 / A = -s c3 (because zr^2 + s q^2 = |1 + i tau|^(2n) = A),
 // so no coefficient is formed by cancellation.
+template <int ORD = 0>
 __device__ __forceinline__ F3 multistep_delta32(F3 v, F3 E, F3 B, float fac, int N, int n) {
     F3 t_n = fac * B;
     F3 e_n = fac * E;
-    float s = dot(t_n, t_n);
+    float s = dot_fma<ORD>(t_n, t_n);
     if (N != 2) {
         float f_N, e_corr;
         if (N == 4) {
@@ -455,7 +492,7 @@ __device__ __forceinline__ F3 multistep_delta32(F3 v, F3 E, F3 B, float fac, int
         float edt = dot(e_n, t_n);
         e_n = f_N * e_n + (e_corr * edt) * t_n;
         t_n = f_N * t_n;
-        s = dot(t_n, t_n);
+        s = dot_fma<ORD == 0 ? 0 : 2>(t_n, t_n);
     }
     float zr = 1.0f, q = 0.0f, A = 1.0f, R = 0.0f;
     for (int k = 0; k < n; ++k) {
@@ -483,16 +520,16 @@ __device__ __forceinline__ float vfac(const BorisArgs& a, double dt) {
 }
 
 // v advanced by one velocity update with factor h (see vfac) and fields (E, B)
-template <bool MULTI>
+template <bool MULTI, int ORD = 0>
 __device__ __forceinline__ CV vel32h(CV v, F3 E, F3 B, const BorisArgs& a, float h) {
-    F3 d = MULTI ? multistep_delta32(v.h, E, B, h, a.order, a.nsub) : boris_delta32(v.h, E, B, h);
+    F3 d = MULTI ? multistep_delta32<ORD>(v.h, E, B, h, a.order, a.nsub) : boris_delta32<ORD>(v.h, E, B, h);
     cv_add(v, d);
     return v;
 }
 
-template <bool MULTI>
+template <bool MULTI, int ORD = 0>
 __device__ __forceinline__ CV vel32(CV v, F3 E, F3 B, const BorisArgs& a, double dt) {
-    return vel32h<MULTI>(v, E, B, a, vfac<MULTI>(a, dt));
+    return vel32h<MULTI, ORD>(v, E, B, a, vfac<MULTI>(a, dt));
 }
 
 // position push x += v dt with dt = dth + dtl (float pair)

@@ -35,6 +35,43 @@ cudaError_t launch_pack_node_table(const void* src, int src_f64, int64_t nodes, 
     return cudaGetLastError();
 }
 
+// The (3, nx, ny, nz) data of E and B, x fastest, into the interleaved float
+// table (E xyz0, B xyz0 per node), z fastest (eb_node): tiles of 32 x 32 nodes
+// in (x, z) turned in shared memory, so that reads and writes are contiguous.
+template <class S>
+__global__ void __launch_bounds__(256) k_pack_eb(const S* E, const S* B, int nx, int ny, int nz, float4* dst) {
+    __shared__ float tile[6][32][33];
+    const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32, lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    for (int y = blockIdx.z; y < ny; y += gridDim.z) {
+        for (int r = row; r < 32; r += 8)
+            if (z0 + r < nz) {
+                const int64_t k = 3 * (x0 + (int64_t)nx * (y + (int64_t)ny * (z0 + r)));
+                const int m = 3 * (nx - x0 < 32 ? nx - x0 : 32);
+                for (int j = lane; j < m; j += 32) {
+                    tile[j % 3][r][j / 3] = (float)E[k + j];
+                    tile[3 + j % 3][r][j / 3] = (float)B[k + j];
+                }
+            }
+        __syncthreads();
+        for (int r = row; r < 32; r += 8)
+            if (x0 + r < nx && z0 + lane < nz) {
+                float4* o = dst + 2 * (z0 + lane + (int64_t)nz * (y + (int64_t)ny * (x0 + r)));
+                o[0] = make_float4(tile[0][lane][r], tile[1][lane][r], tile[2][lane][r], 0.0f);
+                o[1] = make_float4(tile[3][lane][r], tile[4][lane][r], tile[5][lane][r], 0.0f);
+            }
+        __syncthreads();
+    }
+}
+
+cudaError_t launch_pack_eb(const void* E, const void* B, int src_f64, const int32_t n[3], void* dst, cudaStream_t s) {
+    const dim3 grid((n[0] + 31) / 32, (n[2] + 31) / 32, n[1] < 65535 ? n[1] : 65535);
+    if (src_f64)
+        k_pack_eb<double><<<grid, 256, 0, s>>>((const double*)E, (const double*)B, n[0], n[1], n[2], (float4*)dst);
+    else
+        k_pack_eb<float><<<grid, 256, 0, s>>>((const float*)E, (const float*)B, n[0], n[1], n[2], (float4*)dst);
+    return cudaGetLastError();
+}
+
 // slot-major (t[k*n+i], u[(k*W+c)*n+i]) -> per-trajectory packed
 // (t_out[off_i + k], u_out[(off_i + k)*W + c]).  One warp per particle
 // group: threads stride over (particle, save) pairs.

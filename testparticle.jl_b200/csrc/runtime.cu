@@ -65,7 +65,6 @@ struct tp_field {
     void* d_tab32 = nullptr; // float per-node table (only for f64 data)
     // interleaved E/B table built on first use with a partner field
     uint64_t eb_partner = 0;
-    void* d_eb = nullptr;
     void* d_eb32 = nullptr;
     // the same for two cubic periodic grids (k_cubic32c)
     uint64_t ebc_partner = 0;
@@ -487,32 +486,19 @@ int make_dev_fields(tp_ctx* ctx, const tp_field* E, tp_field* B, DevFields& F) {
     F.B = B->dev;
     if (same_geometry(E, B)) {
         if (B->eb_partner != E->id) {
-            if (B->d_eb) cudaFree(B->d_eb);
             if (B->d_eb32) cudaFree(B->d_eb32);
-            B->d_eb = B->d_eb32 = nullptr;
-            bool f64 = B->desc.dtype == TP_DTYPE_F64;
-            size_t esz = f64 ? sizeof(double) : sizeof(float);
-            cudaError_t e = cudaMalloc(&B->d_eb, (size_t)B->nodes * 8 * esz);
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "interleaved field table");
-            e = launch_pack_node_table(E->d_raw, f64, E->nodes, B->d_eb, f64, 2, 0, ctx->stream);
+            B->d_eb32 = nullptr;
+            cudaError_t e = cudaMalloc(&B->d_eb32, (size_t)B->nodes * 8 * sizeof(float));
             if (e == cudaSuccess)
-                e = launch_pack_node_table(B->d_raw, f64, B->nodes, B->d_eb, f64, 2, 1, ctx->stream);
-            if (e == cudaSuccess && f64) {
-                e = cudaMalloc(&B->d_eb32, (size_t)B->nodes * 8 * sizeof(float));
-                if (e == cudaSuccess)
-                    e = launch_pack_node_table(E->d_raw, 1, E->nodes, B->d_eb32, 0, 2, 0, ctx->stream);
-                if (e == cudaSuccess)
-                    e = launch_pack_node_table(B->d_raw, 1, B->nodes, B->d_eb32, 0, 2, 1, ctx->stream);
-            }
+                e = launch_pack_eb(E->d_raw, B->d_raw, B->desc.dtype == TP_DTYPE_F64, B->dev.n, B->d_eb32, ctx->stream);
             // the table is complete before any launch reads it: the entries
             // that take the caller's stream are not ordered after this one
             if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "interleaved field table");
             B->eb_partner = E->id;
         }
-        F.eb = B->d_eb;
         F.eb_f64 = B->desc.dtype == TP_DTYPE_F64;
-        F.eb32 = (const float4*)(B->d_eb32 ? B->d_eb32 : B->d_eb);
+        F.eb32 = (const float4*)B->d_eb32;
     } else if (same_geometry_cubic(E, B)) {
         if (B->ebc_partner != E->id) {
             if (B->d_ebc32) cudaFree(B->d_ebc32);
@@ -571,6 +557,9 @@ void set_wrap(BorisArgs& a, const tp_field* E, const tp_field* B, const tp_term_
             a.wrap[c] = 1;
             a.wrapL[c] = L;
             a.wrap0[c] = x0;
+            a.wrapL32[c] = (float)L;
+            a.wrap0_32[c] = (float)x0;
+            a.wrap1_32[c] = a.wrap0_32[c] + a.wrapL32[c];
         }
     }
     (void)any_grid;
@@ -875,7 +864,7 @@ void tp_field_destroy(tp_field* f) {
     if (!f) return;
     DeviceGuard g(f->ctx->device);
     cudaStreamSynchronize(f->ctx->stream);
-    for (void* p : {f->d_raw, f->d_tab, f->d_tab32, f->d_eb, f->d_eb32, f->d_ebc32, f->d_axis[0], f->d_axis[1], f->d_axis[2],
+    for (void* p : {f->d_raw, f->d_tab, f->d_tab32, f->d_eb32, f->d_ebc32, f->d_axis[0], f->d_axis[1], f->d_axis[2],
                     f->d_snaps, f->d_times, f->d_self})
         if (p) cudaFree(p);
     for (tp_field* c : f->snaps) tp_field_destroy(c);
@@ -2766,8 +2755,8 @@ int adjoint_backward_on(tp_tape* t, const double* gfinal_dev, double* gu0_dev, d
     if (eb) {
         e = launch_table_sum(t->d_geb, t->nodes_B, 2, 0, G, t->d_gparam, s);
         if (e == cudaSuccess) e = launch_table_sum(t->d_geb, t->nodes_B, 2, 1, G, t->d_gparam + 3, s);
-        if (e == cudaSuccess && gE_dev) e = launch_table_unpack(t->d_geb, t->nodes_B, 2, 0, G, gE_dev, s);
-        if (e == cudaSuccess && gB_dev) e = launch_table_unpack(t->d_geb, t->nodes_B, 2, 1, G, gB_dev, s);
+        if (e == cudaSuccess && gE_dev) e = launch_eb_unpack(t->d_geb, t->B->dev.n, 0, G, gE_dev, s);
+        if (e == cudaSuccess && gB_dev) e = launch_eb_unpack(t->d_geb, t->B->dev.n, 1, G, gB_dev, s);
     }
     if (e == cudaSuccess && gridE) {
         e = launch_table_sum(t->d_gE, t->nodes_E, 1, 0, G, t->d_gparam, s);

@@ -1,7 +1,8 @@
-// seg_common.cuh -- the fixed-step and adaptive drivers of the analytic field
-// configurations that have kernels of their own: E zero and B a dipole, or both
-// fields uniform.  Instantiated by boris_seg64.cu (float64) and boris_seg32.cu
-// (FP32C) with the arithmetic as a policy.
+// seg_common.cuh -- the fixed-step and adaptive drivers of the field
+// configurations that have kernels of their own: E zero and B a dipole, both
+// fields uniform, and (fixed steps) E and B on one trilinear grid.  Instantiated
+// by boris_seg64.cu (float64) and boris_seg32.cu (FP32C) with the arithmetic as a
+// policy.
 //
 // The general kernels (k_fixed*, k_adaptive*) decide after every step whether a
 // save, the end, the time budget or a refill is due, and evaluate whatever
@@ -18,7 +19,10 @@
 //   init(a, p, v, u0)              state of a particle
 //   save_first(a, S, i, p, v)      save slot 0 (the initial state)
 //   start(a, dt)                   per-particle constants of a step of length dt
-//   kick(a, p, v, out)             velocity after that step; false: refused
+//   F, fields(a, p)                what a lane evaluates alone at p (may be empty)
+//   kWarp, gather(a, p)            or what the whole warp evaluates together
+//   kick(a, p, v, F, out)          velocity after that step; false: refused
+//   update(a, p, v, F, dt)         one update of any length with those fields
 //   general(a, p, v, dt)           one update of any length by the general functions
 //   advance(a, p, v, dt)           position after the step
 //   outside(a, p, v, t)            termination predicate
@@ -96,12 +100,18 @@ __global__ void __launch_bounds__(PUSH::kBound, 1) k_seg(const __grid_constant__
         }
         bool done = i >= 0 && it > nt;
         // ---- a step that saves, or that the fast functions refused
-        if (i >= 0 && !done && (slow || (a.save_everystep && it > 1 && csave == 0))) {
+        const bool odd = i >= 0 && !done && (slow || (a.save_everystep && it > 1 && csave == 0));
+        typename PUSH::F f;
+        if constexpr (PUSH::kWarp) {
+            if (__any_sync(0xffffffffu, odd)) f = PUSH::gather(a, r);
+        }
+        if (odd) {
             slow = false;
+            if constexpr (!PUSH::kWarp) f = PUSH::fields(a, r);
             const double tn = t + dt;
             typename PUSH::V vn;
-            if (!push.kick(a, r, v, vn)) vn = PUSH::general(a, r, v, dt);
-            const typename PUSH::Pos rn = PUSH::advance(a, r, vn, dt);
+            if (!push.kick(a, r, v, f, vn)) vn = PUSH::general(a, r, v, dt);
+            const typename PUSH::Pos rn = push.advance(a, r, vn, dt);
             if (a.term.flags && PUSH::outside(a, rn, vn, tn + 0.5 * dt)) {
                 done = true;
             } else {
@@ -109,7 +119,7 @@ __global__ void __launch_bounds__(PUSH::kBound, 1) k_seg(const __grid_constant__
                     iout += 1;
                     if (iout <= nout) {
                         t_last = tn - 0.5 * dt;
-                        S.save(i, iout - 1, r, PUSH::general(a, r, v, 0.5 * dt), t_last);
+                        S.save(i, iout - 1, r, PUSH::update(a, r, v, f, 0.5 * dt), t_last);
                     }
                 }
                 r = rn;
@@ -141,15 +151,17 @@ __global__ void __launch_bounds__(PUSH::kBound, 1) k_seg(const __grid_constant__
         // serves the termination rollback
         int taken = 0;
         for (int k = 0; k < len; ++k) {
+            if constexpr (PUSH::kWarp) f = PUSH::gather(a, r);
             if (!go) continue;
+            if constexpr (!PUSH::kWarp) f = PUSH::fields(a, r);
             const double tn = t + dt;
             typename PUSH::V vn;
-            if (!push.kick(a, r, v, vn)) {
+            if (!push.kick(a, r, v, f, vn)) {
                 slow = true;
                 go = false;
                 continue;
             }
-            const typename PUSH::Pos rn = PUSH::advance(a, r, vn, dt);
+            const typename PUSH::Pos rn = push.advance(a, r, vn, dt);
             if (a.term.flags && PUSH::outside(a, rn, vn, tn + 0.5 * dt)) {
                 done = true;
                 go = false;

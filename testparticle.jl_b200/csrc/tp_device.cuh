@@ -89,14 +89,22 @@ __device__ __forceinline__ void quad_eval(const DevField& f, double x, double y,
 
 struct DevFields {
     DevField E, B;
-    const void* eb;   // interleaved table (E xyz0, B xyz0) per node, or null
-    const float4* eb32;   // float interleaved table for the FP32C kernels
+    // E and B on one trilinear grid: the float table with (E xyz0, B xyz0) per
+    // node, z fastest (eb_node), else null; eb_f64: the data are float64, so
+    // only the FP32C kernels read it
+    const float4* eb32;
     int32_t eb_f64;
     int32_t pad;
     // E and B on one periodic, uniform, Cartesian 3-D grid of order 3: their
     // float interleaved table (the warp-cooperative FP32C kernel), else null
     const float4* ebc32;
 };
+
+// node index in the interleaved table: z fastest, so that the two nodes a
+// stencil takes along z share a 128-byte line (pair_gather.cuh)
+__host__ __device__ __forceinline__ int eb_node(const DevField& g, int ix, int iy, int iz) {
+    return iz + g.n[2] * (iy + g.n[1] * ix);
+}
 
 // Termination predicate (the reference's isoutside, as flags).
 struct DevTerm {
@@ -129,7 +137,7 @@ __host__ __device__ __forceinline__ int field_config_of(const DevFields& f) {
         f.E.kind == TP_FIELD_SERIES || f.B.kind == TP_FIELD_SERIES)
         return FK_GENGRID;
     if (f.E.kind == TP_FIELD_QUADRATIC || f.B.kind == TP_FIELD_QUADRATIC) return FK_GENERIC;
-    if (f.eb && !f.eb_f64) return FK_EBGRID;  // float interleaved table
+    if (f.eb32 && !f.eb_f64) return FK_EBGRID;  // float interleaved table
     if (f.E.kind != TP_FIELD_GRID && f.B.kind != TP_FIELD_GRID) return FK_ANALYTIC;
     return FK_GENERIC;
 }
@@ -168,6 +176,7 @@ struct BorisArgs {
     int32_t wrap[3];
     int32_t save_work;    // work rates appended to every save (width + 4)
     double wrapL[3], wrap0[3];
+    float wrapL32[3], wrap0_32[3], wrap1_32[3];  // float period, lower and upper edge
     int32_t ppt;          // particles per thread of the fixed-step kernels (1 or 2)
     int32_t pad_ppt;
     // optional processing order: the k-th particle a kernel takes is perm[k]

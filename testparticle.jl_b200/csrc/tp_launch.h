@@ -162,6 +162,11 @@ cudaError_t launch_table_unpack(const float4* tab, int64_t nodes, int stride, in
 // the kernel of a run that seg_config() accepts (boris_seg64.cu, boris_seg32.cu)
 const void* seg_kernel64(const BorisArgs& a, bool queue);
 const void* seg_kernel32(const BorisArgs& a, bool queue);
+// fixed steps with E and B on one trilinear grid (boris_grid32.cu)
+const void* grid_kernel32(const BorisArgs& a, bool queue);
+// the same for the E (off 0) or B (off 1) half of the interleaved table
+cudaError_t launch_eb_unpack(const float4* tab, const int32_t n[3], int off, int G, double* out, cudaStream_t s);
+
 cudaError_t launch_boris_fp64(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s);
 cudaError_t launch_boris_fp32c(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s);
 // the FP32C run takes the warp-cooperative cubic-grid kernel (static schedule only)
@@ -209,6 +214,8 @@ cudaError_t cell_order(const double* u0, int64_t n, const DevField& g, void* tmp
                        int32_t** perm, cudaStream_t s);
 cudaError_t launch_pack_node_table(const void* src, int src_f64, int64_t nodes, void* dst,
                                    int dst_f64, int stride, int off, cudaStream_t s);
+// E and B data (both float64, or both float32) into the interleaved table
+cudaError_t launch_pack_eb(const void* E, const void* B, int src_f64, const int32_t n[3], void* dst, cudaStream_t s);
 cudaError_t launch_pack_results(const double* t_in, const double* u_in, const int32_t* nsaved,
                                 const int64_t* offsets, int64_t n, int64_t nslots, int width,
                                 double* t_out, double* u_out, cudaStream_t s);
