@@ -798,7 +798,8 @@ static const void* kernel_ptr32(bool adaptive, int ppt) {
     if (adaptive) return (const void*)k_adaptive32c<MULTI, QUEUE, FK>;
     if constexpr (FK == FK_ANALYTIC)
         if (ppt == 2) return (const void*)k_fixed32c_slots<MULTI, QUEUE, FK, 2>;
-    return (const void*)k_fixed32c<MULTI, QUEUE, FK>;
+    if constexpr (FK == FK_EBGRID) return nullptr;  // grid_kernel32
+    else return (const void*)k_fixed32c<MULTI, QUEUE, FK>;
 }
 
 template <bool MULTI, bool QUEUE>

@@ -423,7 +423,8 @@ static const void* kernel_ptr64(bool adaptive, int ppt) {
     if (adaptive) return (const void*)k_adaptive64<MULTI, QUEUE, FK>;
     if constexpr (FK == FK_ANALYTIC)
         if (ppt == 2) return (const void*)k_fixed64_slots<MULTI, QUEUE, FK, 2>;
-    return (const void*)k_fixed64<MULTI, QUEUE, FK>;
+    if constexpr (FK == FK_EBGRID) return nullptr;  // grid_kernel64
+    else return (const void*)k_fixed64<MULTI, QUEUE, FK>;
 }
 
 template <bool MULTI, bool QUEUE>
@@ -437,6 +438,8 @@ static const void* pick_fk64(bool adaptive, const BorisArgs& a) {
 
 static const void* select_kernel64(const BorisArgs& a, bool queue) {
     if (seg_config(a)) return seg_kernel64(a, queue);
+    if (field_config_of(a.f) == FK_EBGRID && (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP))
+        return grid_kernel64(a, queue);
     const bool multi = a.alg == TP_ALG_MULTISTEP || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     if (multi) return queue ? pick_fk64<true, true>(adaptive, a) : pick_fk64<true, false>(adaptive, a);

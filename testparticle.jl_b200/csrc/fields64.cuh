@@ -65,6 +65,28 @@ __device__ __forceinline__ bool grid_axis(const DevField& g, int a, double x, Ax
     return true;
 }
 
+// grid_axis on a periodic axis, without the 64-bit remainder (float64 positions
+// are not wrapped, so most particles leave the box in a long run)
+__device__ __forceinline__ void grid_axis_periodic(const DevField& g, int a, double x, Ax& o) {
+    const double u = (x - g.x0[a]) * g.inv_dx[a];
+    const double fl = floor(u);
+    if (!(fabs(fl) < 4194304.0)) {
+        grid_axis(g, a, x, o);
+        return;
+    }
+    const int na = g.n[a];
+    int i = (int)fl;
+    if ((unsigned)i >= (unsigned)na) {
+        // i / na to the nearest integer, off by less than 1/4 for |i| < 2^22
+        const float q = (float)i * g.inv_n[a] + 12582912.0f;  // 1.5 * 2^23
+        i -= (__float_as_int(q) - __float_as_int(12582912.0f)) * na;
+        if (i < 0) i += na;
+    }
+    o.f = u - fl;
+    o.i0 = i;
+    o.i1 = (i + 1 == na) ? 0 : i + 1;
+}
+
 __device__ __forceinline__ double lerp64(double a, double b, double f) { return a + f * (b - a); }
 
 // Load node `node` of a table with `stride` 4-vectors per node, at offset `off`.
@@ -383,8 +405,8 @@ __device__ __forceinline__ D3 multistep_rot64(D3 v, D3 E, D3 B, double q2m, doub
     return out;
 }
 
-// ---------------------------------------------------------------- E zero, B a dipole (FK_DIPOLE)
-// The arithmetic of analytic_eval64 / boris_rot64 / multistep_rot64 with the
+// ---------------------------------------------------------------- updates of the segment kernels
+// E zero, B a dipole (FK_DIPOLE): the arithmetic of analytic_eval64 / boris_rot64 / multistep_rot64 with the
 // shared reciprocals of fdiv64.cuh and without the terms of a zero E: 237
 // float64-pipe instructions per Multistep step instead of 358.  The float64
 // pipe (16 lanes per sub-partition) is what bounds these kernels.  They return
@@ -407,7 +429,21 @@ __device__ __forceinline__ bool dipole_fast64(const DevField& f, D3 r, D3& B) {
     return true;
 }
 
-// boris_rot64 with E zero; qdt = q2m * 0.5 * dt
+// boris_rot64; qdt = q2m * 0.5 * dt
+__device__ __forceinline__ bool boris_fast64(D3 v, D3 E, D3 B, double qdt, D3& out) {
+    const D3 t = qdt * B;
+    const double b = 1.0 + abs2sum(t);
+    if (!in_range64(b) && !isnan(b)) return false;
+    const Rec64 q = rec64(b, rcp64(b));
+    const D3 s{quot64(2.0 * t.x, q), quot64(2.0 * t.y, q), quot64(2.0 * t.z, q)};
+    const D3 he = qdt * E;
+    const D3 vm = v + he;
+    const D3 vp = vm + cross(vm, t);
+    out = (vm + cross(vp, s)) + he;
+    return true;
+}
+
+// the same with E zero
 __device__ __forceinline__ bool boris_fast64(D3 v, D3 B, double qdt, D3& out) {
     const D3 t = qdt * B;
     const double b = 1.0 + abs2sum(t);

@@ -358,6 +358,7 @@ void fill_float_copies(DevField& d) {
         d.x0f[a] = (float)d.x0[a];
         d.dxf[a] = (float)(1.0 / d.inv_dx[a]);
         d.idxf[a] = (float)d.inv_dx[a];
+        d.inv_n[a] = d.n[a] > 0 ? 1.0f / (float)d.n[a] : 0.0f;
     }
     for (int k = 0; k < 9; ++k) d.Jf[k] = (float)d.J[k];
     d.coeff = (float)d.coef;

@@ -36,6 +36,7 @@ struct DevField {
     double x0[3];
     double inv_dx[3];
     double L[3];      // periodic length n*dx
+    float inv_n[3];   // 1 / n
     float x0f[3];     // float copies for the FP32C kernels
     float dxf[3];
     float idxf[3];

@@ -162,7 +162,8 @@ cudaError_t launch_table_unpack(const float4* tab, int64_t nodes, int stride, in
 // the kernel of a run that seg_config() accepts (boris_seg64.cu, boris_seg32.cu)
 const void* seg_kernel64(const BorisArgs& a, bool queue);
 const void* seg_kernel32(const BorisArgs& a, bool queue);
-// fixed steps with E and B on one trilinear grid (boris_grid32.cu)
+// fixed steps with E and B on one trilinear grid (boris_grid64.cu, boris_grid32.cu)
+const void* grid_kernel64(const BorisArgs& a, bool queue);
 const void* grid_kernel32(const BorisArgs& a, bool queue);
 // the same for the E (off 0) or B (off 1) half of the interleaved table
 cudaError_t launch_eb_unpack(const float4* tab, const int32_t n[3], int off, int G, double* out, cudaStream_t s);
