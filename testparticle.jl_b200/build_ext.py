@@ -1,8 +1,8 @@
 """Build libtpb200.so (the CUDA library behind include/tp_abi.h) in-tree.
 
 Every translation unit is compiled for sm_100a only.  The float64 kernels
-(boris_fp64.cu, boris_seg64.cu, boris_grid64.cu, gc_fp64.cu, hybrid.cu,
-detect.cu) are compiled with -fmad=false so that their arithmetic follows the
+(boris_fp64.cu, boris_seg64.cu, boris_grid64.cu, gc_fp64.cu, gc_dipole64.cu,
+hybrid.cu, detect.cu) are compiled with -fmad=false so that their arithmetic follows the
 reference's operation order; the float32 kernels use contraction.  Objects are rebuilt only when a source or header is newer.
 """
 from __future__ import annotations
@@ -22,10 +22,10 @@ INCLUDE = HERE.parent / "include"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
           "--expt-relaxed-constexpr", f"-I{INCLUDE}", f"-I{CSRC}"]
-NO_FMAD = {"boris_fp64.cu", "boris_seg64.cu", "boris_grid64.cu", "gc_fp64.cu", "hybrid.cu", "detect.cu"}
+NO_FMAD = {"boris_fp64.cu", "boris_seg64.cu", "boris_grid64.cu", "gc_fp64.cu", "gc_dipole64.cu", "hybrid.cu", "detect.cu"}
 SOURCES = ["runtime.cu", "pack.cu", "boris_fp64.cu", "boris_seg64.cu", "boris_grid64.cu", "boris_fp32c.cu",
-           "boris_seg32.cu", "boris_grid32.cu", "gc_fp64.cu", "gc_fp32.cu", "adjoint.cu", "noalloc.cu", "hybrid.cu",
-           "detect.cu"]
+           "boris_seg32.cu", "boris_grid32.cu", "gc_fp64.cu", "gc_dipole64.cu", "gc_fp32.cu", "adjoint.cu", "noalloc.cu",
+           "hybrid.cu", "detect.cu"]
 
 
 def _nvcc() -> str:

@@ -37,9 +37,16 @@ __host__ __device__ __forceinline__ int gc_grid_mode(const DevFields& f) {
     return (ge || gb || quad) ? GM_GRID : GM_ANALYTIC;
 }
 
+//
+// A right-hand side class has the grid mode kGM, register caps for the two
+// drivers (threads), start(p), called once per particle, and kFast: it computes
+// in a restricted range and clears ok outside it, upon which the driver repeats
+// the step with RHS64 (step_general).
 template <int GM>
 struct RHS64 {
-    static constexpr int kGM = GM;
+    static constexpr int kGM = GM, kRk4Bound = 256, kRk45Bound = 384;
+    static constexpr bool kFast = false;
+    __device__ __forceinline__ void start(const GCPar&) {}
     __device__ __forceinline__ G4 operator()(const DevFields& F, const G4& s, const GCPar& p,
                                              double t) const {
         D3 X{s.y[0], s.y[1], s.y[2]};
@@ -129,7 +136,7 @@ __device__ __forceinline__ int64_t gc_next(const GCArgs& a, int64_t& first) {
 // unrolled (the right-hand side inlined once, as in update_dp5); the sum
 // ((k1 + 2 k2) + 2 k3) + k4 is accumulated in the reference's order.
 template <class RHS>
-__device__ __forceinline__ G4 update_rk4(const RHS& f, const DevFields& F, const G4& y,
+__device__ __forceinline__ G4 update_rk4(RHS& f, const DevFields& F, const G4& y,
                                          const GCPar& p, double dt, double t) {
     G4 k = f(F, y, p, t);
     G4 sum = k;
@@ -143,9 +150,15 @@ __device__ __forceinline__ G4 update_rk4(const RHS& f, const DevFields& F, const
     return gscale(dt / 6.0, sum);
 }
 
+// one step with the general float64 right-hand side (analytic fields)
+static __device__ __noinline__ G4 rk4_general(const GCArgs& a, G4 y, GCPar p, double dt, double t) {
+    RHS64<GM_ANALYTIC> f;
+    return update_rk4(f, a.f, y, p, dt, t);
+}
+
 template <class RHS, bool QUEUE>
-__global__ void __launch_bounds__(256) k_rk4(GCArgs a) {
-    const RHS f;
+__global__ void __launch_bounds__(RHS::kRk4Bound, 1) k_rk4(const __grid_constant__ GCArgs a) {
+    RHS f;
     const GCSaver<RHS::kGM> S(a);
     const uint64_t t_start = globaltimer_ns();
     int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -159,6 +172,7 @@ __global__ void __launch_bounds__(256) k_rk4(GCArgs a) {
             i = gc_next<QUEUE>(a, first);
             if (i >= a.n) break;
             p = gc_par(a, i);
+            f.start(p);
             const double* y0 = a.y0 + 4 * i;
             xv = {{y0[0], y0[1], y0[2], y0[3]}};
             dt = a.dt_i ? a.dt_i[i] : a.dt;
@@ -194,6 +208,10 @@ __global__ void __launch_bounds__(256) k_rk4(GCArgs a) {
         if (!done) {
             double t = fma((double)(it - 1), dt, a.t0);
             G4 dx = update_rk4(f, a.f, xv, p, dt, t);
+            if constexpr (RHS::kFast) {
+                if (!f.ok) dx = rk4_general(a, xv, p, dt, t);
+                f.ok = true;
+            }
             G4 xn = gadd(xv, dx);
             if (a.term.flags && outside_gc(a.term, xn, t + dt)) {
                 done = true;
@@ -290,7 +308,7 @@ __constant__ const DP5Tableau kDP5 = {
     {0.0, 1.0 / 5, 3.0 / 10, 4.0 / 5, 8.0 / 9, 1.0, 1.0}};
 
 template <class RHS>
-__device__ __forceinline__ void update_dp5(const RHS& f, const DevFields& F, const G4& y,
+__device__ __forceinline__ void update_dp5(RHS& f, const DevFields& F, const G4& y,
                                            const GCPar& p, double dt, double t, const G4& k1, G4& dy, G4& err,
                                            G4& y7, G4& k7) {
     const double b1 = 35.0 / 384, b3 = 500.0 / 1113, b4 = 125.0 / 192, b5 = -2187.0 / 6784,
@@ -318,11 +336,23 @@ __device__ __forceinline__ void update_dp5(const RHS& f, const DevFields& F, con
                           gscale(e7, k[6])));
 }
 
-// Register cap 168 (65536 / 384): three blocks of 128 threads per SM for the
-// float64 right-hand side instead of two, for a few bytes of spill.
+// one attempt with the general float64 right-hand side (analytic fields), k1 included
+struct DP5Step {
+    G4 k1, dx, E, y7, k7;
+};
+static __device__ __noinline__ DP5Step dp5_general(const GCArgs& a, G4 y, GCPar p, double dt, double t, bool have_k1, G4 k1) {
+    RHS64<GM_ANALYTIC> f;
+    DP5Step s;
+    s.k1 = have_k1 ? k1 : f(a.f, y, p, t);
+    update_dp5(f, a.f, y, p, dt, t, s.k1, s.dx, s.E, s.y7, s.k7);
+    return s;
+}
+
+// Register cap of the general right-hand sides 168 (65536 / 384): three blocks of
+// 128 threads per SM in float64 instead of two, for a few bytes of spill.
 template <class RHS, bool QUEUE>
-__global__ void __launch_bounds__(384, 1) k_rk45(GCArgs a) {
-    const RHS f;
+__global__ void __launch_bounds__(RHS::kRk45Bound, 1) k_rk45(const __grid_constant__ GCArgs a) {
+    RHS f;
     const GCSaver<RHS::kGM> S(a);
     const uint64_t t_start = globaltimer_ns();
     int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -338,6 +368,7 @@ __global__ void __launch_bounds__(384, 1) k_rk45(GCArgs a) {
             i = gc_next<QUEUE>(a, first);
             if (i >= a.n) break;
             p = gc_par(a, i);
+            f.start(p);
             const double* y0 = a.y0 + 4 * i;
             xv = {{y0[0], y0[1], y0[2], y0[3]}};
             t = a.t0;
@@ -377,6 +408,17 @@ __global__ void __launch_bounds__(384, 1) k_rk45(GCArgs a) {
             if (!have_k1) k1 = f(a.f, xv, p, t);
             G4 dx, E, y7, k7;
             update_dp5(f, a.f, xv, p, dt, t, k1, dx, E, y7, k7);
+            if constexpr (RHS::kFast) {
+                if (!f.ok) {
+                    const DP5Step s = dp5_general(a, xv, p, dt, t, have_k1, k1);
+                    k1 = s.k1;
+                    dx = s.dx;
+                    E = s.E;
+                    y7 = s.y7;
+                    k7 = s.k7;
+                }
+                f.ok = true;
+            }
             G4 yn = gadd(xv, dx);
             have_k1 = true;
             double sum_sq = 0.0;

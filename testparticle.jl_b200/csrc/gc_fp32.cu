@@ -73,7 +73,9 @@ __device__ __forceinline__ void field_jac32(const DevField& f, V3f r, float t, V
 
 template <int GM>
 struct RHS32 {
-    static constexpr int kGM = GM;
+    static constexpr int kGM = GM, kRk4Bound = 256, kRk45Bound = 384;
+    static constexpr bool kFast = false;
+    __device__ __forceinline__ void start(const GCPar&) {}
     __device__ __forceinline__ G4 operator()(const DevFields& F, const G4& s, const GCPar& p,
                                              double t) const {
         V3f E, B;

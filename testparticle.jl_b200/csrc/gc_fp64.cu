@@ -120,6 +120,7 @@ static const void* gc_kernel(bool rk4, bool queue) {
 }
 
 const void* select_gc_kernel64(const GCArgs& a, bool queue) {
+    if (const void* k = gc_dipole_kernel64(a, queue)) return k;
     const int gm = gc_grid_mode(a.f);
     bool rk4 = a.alg == TP_GC_RK4;
     if (gm == GM_ANY) return gc_kernel<RHS64<GM_ANY>>(rk4, queue);

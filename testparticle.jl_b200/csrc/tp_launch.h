@@ -175,6 +175,7 @@ bool fp32c_cubic_coop(const BorisArgs& a);
 int occupancy_boris_fp64(const BorisArgs& a, int block);
 int occupancy_boris_fp32c(const BorisArgs& a, int block);
 
+const void* gc_dipole_kernel64(const GCArgs& a, bool queue);
 cudaError_t launch_gc(const GCArgs& a, const LaunchCfg& c, cudaStream_t s);
 cudaError_t launch_gc_fp32(const GCArgs& a, const LaunchCfg& c, cudaStream_t s);
 int occupancy_gc(const GCArgs& a, int block);
