@@ -3,7 +3,8 @@
 // (pair_gather.cuh).  The arithmetic is that of Vel32<FK_EBGRID>.
 //
 // Measured on the 128^3 turbulent field, 1e6 protons, device time: 250 steps 8.43
-// -> 5.71 ms, 1000 steps 31.9 -> 22.3 ms (4.5e10 particle-steps/s).  What bounds it
+// -> 5.37 ms (4.7e10 particle-steps/s), 5.71 while the particles were still sorted by
+// cell first.  What bounds it
 // is the L1 cache (88 % busy): 5 line look-ups per particle and step, 11 shuffles
 // per warp, and the 8 sectors that come from L2.
 #include "boris32_common.cuh"
@@ -29,7 +30,7 @@ __device__ __forceinline__ CV kick_grid32(const BorisArgs& a, CPos p, CV v, doub
 
 template <bool MULTI, bool PERIODIC>
 struct GridPush32 {
-    // register cap (threads), 250 steps of the ensemble above: 384 (165 registers)
+    // register cap (threads), 250 steps of the ensemble above, sorted: 384 (165 registers)
     // 7.17 ms, 512 6.40, 640 5.99, 768 (80) 5.72, 896 5.78
     static constexpr int kBound = 768;
     using Pos = CPos;
@@ -77,8 +78,8 @@ struct GridPush32 {
         out = vel32h<MULTI, kStep>(v, f.E, f.B, a, h);
         return true;
     }
-    static __device__ __forceinline__ CV update(const BorisArgs& a, const CPos&, const CV& v, const F& f, double dt) {
-        return vel32<MULTI, kSave>(v, f.E, f.B, a, dt);
+    __device__ __forceinline__ CV half(const BorisArgs& a, const CPos&, const CV& v, const F& f, double dt) const {
+        return vel32<MULTI, kSave>(v, f.E, f.B, a, 0.5 * dt);
     }
     static __device__ __forceinline__ CV general(const BorisArgs& a, const CPos& p, const CV& v, double dt) {
         return kick_grid32<MULTI>(a, p, v, dt);

@@ -4,7 +4,8 @@
 // results equal those of eb_eval64_f32 and vel_update64 bit for bit.
 //
 // Measured on the device, 400009 protons x 250 steps on a 120 x 100 x 91 grid:
-// Boris 4.72 -> 2.79 ms, MultistepBoris4(2) 6.42 -> 4.07 ms.  A Boris step is 457
+// Boris 4.72 -> 2.55 ms, MultistepBoris4(2) 6.42 -> 4.07 ms (2.79 while the
+// particles were still sorted by cell first).  A Boris step is 457
 // warp instructions, 206 on the float64 pipe and 58 on the XU (float to float64
 // conversions); L1 is 70 % busy with 5 line look-ups per particle.
 #include "boris64_common.cuh"
@@ -15,7 +16,7 @@ namespace tpb {
 
 template <bool MULTI, bool PERIODIC>
 struct GridPush64 {
-    // register cap (threads), 250 steps of the first ensemble above: 384 3.42 ms,
+    // register cap (threads), 250 Boris steps of the ensemble above, sorted: 384 3.42 ms,
     // 512 3.00, 640 (96 registers) 2.79, 768 3.49, 1024 4.59 (spills in the loop)
     static constexpr int kBound = 640;
     using Pos = D3;
@@ -61,8 +62,8 @@ struct GridPush64 {
         out = multistep_rot64(v, f.E, f.B, a.q2m, h, a.order, a.nsub);
         return true;
     }
-    static __device__ __forceinline__ D3 update(const BorisArgs& a, D3, D3 v, const F& f, double dt) {
-        return vel_update64<MULTI>(v, f.E, f.B, a.q2m, dt, a.order, a.nsub);
+    __device__ __forceinline__ D3 half(const BorisArgs& a, D3, D3 v, const F& f, double dt) const {
+        return vel_update64<MULTI>(v, f.E, f.B, a.q2m, 0.5 * dt, a.order, a.nsub);
     }
     static __device__ __forceinline__ D3 general(const BorisArgs& a, D3 r, D3 v, double dt) {
         D3 E, B;

@@ -40,8 +40,8 @@ struct Push32 {
     struct F {};
     static constexpr bool kWarp = false;
     static __device__ __forceinline__ F fields(const BorisArgs&, const CPos&) { return {}; }
-    static __device__ __forceinline__ D3 update(const BorisArgs& a, const CPos& p, D3 v, F, double dt) {
-        return kick_general32<MULTI>(a, p, v, dt);
+    __device__ __forceinline__ D3 half(const BorisArgs& a, const CPos& p, D3 v, F, double dt) const {
+        return kick_general32<MULTI>(a, p, v, 0.5 * dt);
     }
     static __device__ __forceinline__ CPos advance(const BorisArgs& a, CPos p, D3 v, double dt) {
         cpos_push_d(a, p, v, dt);
@@ -63,9 +63,18 @@ struct DipolePush32 : Push32<MULTI> {
     __device__ __forceinline__ void start(const BorisArgs& a, double dt) {
         h = MULTI ? a.q2m * dt / (double)(2 * a.nsub) : a.q2m * 0.5 * dt;
     }
-    __device__ __forceinline__ bool kick(const BorisArgs& a, const CPos& p, D3 v, typename Push32<MULTI>::F, D3& out) const {
-        out = rot_mixed(v, D3{0.0, 0.0, 0.0}, dipole_mixed(a.f.B, p), h, ORD, MULTI ? a.nsub : 1, false);
+    using F = D3;  // B
+    static __device__ __forceinline__ D3 fields(const BorisArgs& a, const CPos& p) { return dipole_mixed(a.f.B, p); }
+    __device__ __forceinline__ D3 rotate(const BorisArgs& a, D3 v, D3 B, double hh) const {
+        return rot_mixed(v, D3{0.0, 0.0, 0.0}, B, hh, ORD, MULTI ? a.nsub : 1, false);
+    }
+    __device__ __forceinline__ bool kick(const BorisArgs& a, const CPos&, D3 v, D3 B, D3& out) const {
+        out = rotate(a, v, B, h);
         return true;
+    }
+    // half the factor is the factor of half the step, exactly
+    __device__ __forceinline__ D3 half(const BorisArgs& a, const CPos&, D3 v, D3 B, double) const {
+        return rotate(a, v, B, 0.5 * h);
     }
     // adaptive steps
     using Bv = D3;

@@ -41,8 +41,8 @@ struct Push64 {
     struct F {};
     static constexpr bool kWarp = false;
     static __device__ __forceinline__ F fields(const BorisArgs&, D3) { return {}; }
-    static __device__ __forceinline__ D3 update(const BorisArgs& a, D3 r, D3 v, F, double dt) {
-        return kick_general64<MULTI>(a, r, v, dt);
+    __device__ __forceinline__ D3 half(const BorisArgs& a, D3 r, D3 v, F, double dt) const {
+        return kick_general64<MULTI>(a, r, v, 0.5 * dt);
     }
     static __device__ __forceinline__ D3 advance(const BorisArgs&, D3 r, D3 v, double dt) { return r + v * dt; }
     static __device__ __forceinline__ bool outside(const BorisArgs& a, D3 r, D3 v, double t) {
@@ -61,10 +61,25 @@ struct DipolePush64 : Push64<MULTI> {
     __device__ __forceinline__ void start(const BorisArgs& a, double dt) {
         h = MULTI ? a.q2m * dt / (double)(2 * a.nsub) : a.q2m * 0.5 * dt;
     }
-    __device__ __forceinline__ bool kick(const BorisArgs& a, D3 r, D3 v, typename Push64<MULTI>::F, D3& out) const {
+    struct F {
         D3 B;
-        return dipole_fast64(a.f.B, r, B) &&
-               (MULTI ? multistep_fast64<ORD>(v, B, h, a.nsub, out) : boris_fast64(v, B, h, out));
+        bool ok;
+    };
+    static __device__ __forceinline__ F fields(const BorisArgs& a, D3 r) {
+        F f;
+        f.ok = dipole_fast64(a.f.B, r, f.B);
+        return f;
+    }
+    __device__ __forceinline__ bool fast(const BorisArgs& a, D3 v, const F& f, double hh, D3& out) const {
+        return f.ok && (MULTI ? multistep_fast64<ORD>(v, f.B, hh, a.nsub, out) : boris_fast64(v, f.B, hh, out));
+    }
+    __device__ __forceinline__ bool kick(const BorisArgs& a, D3, D3 v, const F& f, D3& out) const {
+        return fast(a, v, f, h, out);
+    }
+    // half the factor is the factor of half the step, exactly
+    __device__ __forceinline__ D3 half(const BorisArgs& a, D3 r, D3 v, const F& f, double dt) const {
+        D3 out;
+        return fast(a, v, f, 0.5 * h, out) ? out : kick_general64<MULTI>(a, r, v, 0.5 * dt);
     }
     // adaptive steps
     using Bv = D3;
@@ -96,18 +111,26 @@ template <>
 struct UniformPush64<false> : Push64<false> {
     static constexpr int kBound = TPB_MAXT(FK_ANALYTIC);
     D3 t, s, he;
+    D3 s2;  // s of half a step, whose t and he are half of these
     __device__ __forceinline__ void start(const BorisArgs& a, double dt) {
         const D3 z{0.0, 0.0, 0.0};
         const double h = a.q2m * 0.5 * dt;
         t = h * analytic_eval64(a.f.B, z, 0.0);
         s = (2.0 * t) / (1.0 + abs2sum(t));
+        s2 = t / (1.0 + abs2sum(0.5 * t));
         he = h * analytic_eval64(a.f.E, z, 0.0);
     }
     __device__ __forceinline__ bool kick(const BorisArgs&, D3, D3 v, F, D3& out) const {
+        out = rotate(v, t, s, he);
+        return true;
+    }
+    __device__ __forceinline__ D3 half(const BorisArgs&, D3, D3 v, F, double) const {
+        return rotate(v, 0.5 * t, s2, 0.5 * he);
+    }
+    static __device__ __forceinline__ D3 rotate(D3 v, D3 t, D3 s, D3 he) {
         const D3 vm = v + he;
         const D3 vp = vm + cross(vm, t);
-        out = (vm + cross(vp, s)) + he;
-        return true;
+        return (vm + cross(vp, s)) + he;
     }
 };
 

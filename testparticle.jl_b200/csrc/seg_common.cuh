@@ -22,7 +22,7 @@
 //   F, fields(a, p)                what a lane evaluates alone at p (may be empty)
 //   kWarp, gather(a, p)            or what the whole warp evaluates together
 //   kick(a, p, v, F, out)          velocity after that step; false: refused
-//   update(a, p, v, F, dt)         one update of any length with those fields
+//   half(a, p, v, F, dt)           one update of length dt / 2 with those fields
 //   general(a, p, v, dt)           one update of any length by the general functions
 //   advance(a, p, v, dt)           position after the step
 //   outside(a, p, v, t)            termination predicate
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(PUSH::kBound, 1) k_seg(const __grid_constant__
                     iout += 1;
                     if (iout <= nout) {
                         t_last = tn - 0.5 * dt;
-                        S.save(i, iout - 1, r, PUSH::update(a, r, v, f, 0.5 * dt), t_last);
+                        S.save(i, iout - 1, r, push.half(a, r, v, f, dt), t_last);
                     }
                 }
                 r = rn;
