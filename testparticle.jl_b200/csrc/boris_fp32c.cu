@@ -352,21 +352,26 @@ __global__ void __launch_bounds__(TPB_MAXT(FK) / PPT, 1) k_fixed32c_slots(BorisA
 // 3 (cardinal_interp, src/utility/interpolation.jl:142; the local cubic
 // Hermite with Catmull-Rom slopes of grid_general.cuh), from the interleaved
 // float table (E xyz0, B xyz0 per node, 32 bytes).  A particle's stencil is
-// 4 x 4 x 4 nodes; a row of 4 nodes along x is 128 contiguous bytes.  Instead
-// of each lane gathering its own 64 nodes (64 scattered lines per lane), the
-// warp gathers the stencils of its particles four at a time: for each, lane
-// l loads nodes (l & 3, (l >> 2) & 3, l >> 4) and (.., .., (l >> 4) + 2) -- 8
-// rows of 128 bytes per load instruction -- and weights them; one
-// reduce-scatter over the warp sums the four particles' E and B (reduce4x6)
-// and the owning lanes fetch theirs.  All 32 lanes of the warp must call it
-// together; lanes with want = false only help.
+// 4 x 4 x 4 nodes; a row of 4 nodes along x is 128 contiguous bytes.  Four
+// lanes work on one particle: lane d of the group loads node d of each of the
+// 16 rows (one 256-bit load per row, so a load instruction reads 8 rows of 128
+// bytes), weights and sums its 16 nodes in registers, and two butterfly steps
+// add the four lanes.  A group takes its four particles in turn.  All 32 lanes
+// of the warp must call it together; lanes with want = false only help.
+//
+// The sums keep the order of an earlier form in which the whole warp worked on
+// one particle (z pairs 0,2 and 1,3; then z; then y pairs 0,2 and 1,3; then y;
+// then x), so the results are the same.  That form took 5957 warp instructions
+// per step, most of them index arithmetic, weights and shuffles repeated for
+// every particle by all 32 lanes; this one takes 1850.  Measured: 200000 protons x
+// 200 steps on a 96^3 grid 11.6 -> 4.7 ms, 1e6 x 50 on 128^3 6.1 ms (8.2e9
+// particle-steps/s).  What bounds it now is the path from L2: 64 sectors of 32
+// bytes per particle and step, at 64 bytes per SM and clock 9.1e9.
 // The weight of node d (0..3) of the 4-node stencil at fraction t of the
 // middle cell, w_d(t) = h-basis combination of the Catmull-Rom Hermite cubic
 // (grid_general.cuh), as the polynomial c0 + c1 t + c2 t^2 + c3 t^3:
 //   w0 = -t/2 + t^2 - t^3/2        w1 = 1 - 5t^2/2 + 3t^3/2
 //   w2 =  t/2 + 2t^2 - 3t^3/2      w3 = -t^2/2 + t^3/2
-// A lane always takes the same node of every stencil, so its coefficients
-// are fixed for the whole kernel and a weight costs three FMAs.
 struct CubicW {
     float c0, c1, c2, c3;
 };
@@ -379,129 +384,75 @@ __device__ __forceinline__ float cubic_w(const CubicW& c, float t) {
     return fmaf(fmaf(fmaf(c.c3, t, c.c2), t, c.c1), t, c.c0);
 }
 
-// cell index in [0, n) and fraction in [0, 1) on a periodic axis, from the
-// compensated coordinate (positions are wrapped into the box)
-__device__ __forceinline__ void cubic_cell(const DevField& g, int a, float hi, float lo, int& i, float& f) {
-    AxF o;
-    axis32(g, a, hi, lo, o);  // periodic: always in range
-    i = o.i0;
-    f = o.f;
-}
-
-// this lane's weighted share of the stencil of the particle at cell (qi, qj,
-// qk), fractions (fx, fy, fz): E in s[0..2], B in s[3..5]
-__device__ __forceinline__ void cubic_share(const DevField& g, const float4* tab, int qi, int qj, int qk, float fx,
-                                            float fy, float fz, float s[6]) {
-    const int lane = threadIdx.x & 31;
-    const int dx = lane & 3, dy = (lane >> 2) & 3, dz = lane >> 4;
-    const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-    const float wxy = cubic_w(cubic_coef(dx), fx) * cubic_w(cubic_coef(dy), fy);
-    const float w0 = wxy * cubic_w(cubic_coef(dz), fz), w1 = wxy * cubic_w(cubic_coef(dz + 2), fz);
-    int ix = qi - 1 + dx, iy = qj - 1 + dy, iz0 = qk - 1 + dz, iz1 = qk + 1 + dz;
-    ix += ix < 0 ? nx : 0;
-    ix -= ix >= nx ? nx : 0;
-    iy += iy < 0 ? ny : 0;
-    iy -= iy >= ny ? ny : 0;
-    iz0 += iz0 < 0 ? nz : 0;
-    iz1 -= iz1 >= nz ? nz : 0;
-    const int64_t row = (int64_t)ix + (int64_t)nx * iy;
-    const int64_t nxy = (int64_t)nx * ny;
-    float4 e0, b0, e1, b1;
-    ldg_node8(tab + 2 * (row + nxy * iz0), e0, b0);
-    ldg_node8(tab + 2 * (row + nxy * iz1), e1, b1);
-    s[0] = fmaf(w0, e0.x, w1 * e1.x);
-    s[1] = fmaf(w0, e0.y, w1 * e1.y);
-    s[2] = fmaf(w0, e0.z, w1 * e1.z);
-    s[3] = fmaf(w0, b0.x, w1 * b1.x);
-    s[4] = fmaf(w0, b0.y, w1 * b1.y);
-    s[5] = fmaf(w0, b0.z, w1 * b1.z);
-}
-
-// Sum s[k][c] (particle k = 0..3, component c = 0..5: E xyz, B xyz) over the
-// 32 lanes of the warp by halving (a reduce-scatter): after the exchanges with
-// lanes 16, 8 and 4 apart each lane holds three components of one particle
-// summed over 8 lanes -- particle 2 b4 + b3, components 3 b2 .. 3 b2 + 2 for
-// lane bits b4 b3 b2 -- and two butterfly levels complete the sums: 27
-// shuffles for four particles instead of 120.  Returns the three sums.
-__device__ __forceinline__ void reduce4x6(const float s[4][6], float out[3]) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const bool b4 = (lane >> 4) & 1, b3 = (lane >> 3) & 1, b2 = (lane >> 2) & 1;
-    // lanes 16 apart: keep particles {0, 1} (b4 = 0) or {2, 3}
-    float t[2][6];
+// one row pair of the stencil at y offset `oy`: the lane's nodes at the four z
+// offsets, weighted by wxy and wz and summed over z
+__device__ __forceinline__ void cubic_rows(const float4* tab, int oy, const int oz[4], float wxy, const float wz[4],
+                                           float s[6]) {
+    float4 e[4], b[4];
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            const float keep = b4 ? s[2 + k][c] : s[k][c];
-            const float send = b4 ? s[k][c] : s[2 + k][c];
-            t[k][c] = keep + __shfl_xor_sync(full, send, 16);
-        }
-    // lanes 8 apart: keep particle b3 of the pair
-    float u[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        const float keep = b3 ? t[1][c] : t[0][c];
-        const float send = b3 ? t[0][c] : t[1][c];
-        u[c] = keep + __shfl_xor_sync(full, send, 8);
-    }
-    // lanes 4 apart: keep E (b2 = 0) or B
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const float keep = b2 ? u[3 + c] : u[c];
-        const float send = b2 ? u[c] : u[3 + c];
-        out[c] = keep + __shfl_xor_sync(full, send, 4);
-    }
-#pragma unroll
-    for (int o = 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) out[c] += __shfl_xor_sync(full, out[c], o);
+    for (int k = 0; k < 4; ++k) ldg_node8(tab + 2 * (int64_t)(oy + oz[k]), e[k], b[k]);
+    const float w0 = wxy * wz[0], w1 = wxy * wz[1], w2 = wxy * wz[2], w3 = wxy * wz[3];
+#define TPB_ZSUM(q, c) __fadd_rn(fmaf(w0, q[0].c, w2 * q[2].c), fmaf(w1, q[1].c, w3 * q[3].c))
+    s[0] = TPB_ZSUM(e, x);
+    s[1] = TPB_ZSUM(e, y);
+    s[2] = TPB_ZSUM(e, z);
+    s[3] = TPB_ZSUM(b, x);
+    s[4] = TPB_ZSUM(b, y);
+    s[5] = TPB_ZSUM(b, z);
+#undef TPB_ZSUM
 }
 
 __device__ __forceinline__ void coop_cubic_eval(const DevField& g, const float4* tab, bool want, const CPos& p,
                                                 F3& E, F3& B) {
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    int ci[3] = {0, 0, 0};
-    float cf[3] = {0.0f, 0.0f, 0.0f};
-    if (want) {
-        cubic_cell(g, 0, p.hi[0], p.lo[0], ci[0], cf[0]);
-        cubic_cell(g, 1, p.hi[1], p.lo[1], ci[1], cf[1]);
-        cubic_cell(g, 2, p.hi[2], p.lo[2], ci[2], cf[2]);
-    }
-    unsigned mask = __ballot_sync(full, want);
-    // four particles per round (the last round repeats its final particle)
-    while (mask) {
-        int q[4];
-        q[0] = __ffs(mask) - 1;
-        mask &= mask - 1;
+    const int d = threadIdx.x & 3;
+    const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
+    AxF ax{}, ay{}, az{};
+    if (want) axes32(g, p, ax, ay, az);  // periodic: always in range
+    const unsigned mask = __ballot_sync(full, want);
+    const CubicW cx = cubic_coef(d);
+#pragma unroll 1
+    for (int r = 0; r < 4; ++r) {
+        if (!(mask & (0x11111111u << r))) continue;  // warp-uniform
+        const int src = (threadIdx.x & 28) | r;
+        const int qi = __shfl_sync(full, ax.i0, src), qj = __shfl_sync(full, ay.i0, src), qk = __shfl_sync(full, az.i0, src);
+        const float fx = __shfl_sync(full, ax.f, src), fy = __shfl_sync(full, ay.f, src), fz = __shfl_sync(full, az.f, src);
+        int ix = qi - 1 + d;
+        ix += ix < 0 ? nx : 0;
+        ix -= ix >= nx ? nx : 0;
+        int oy[4], oz[4];
+        float wz[4];
 #pragma unroll
-        for (int k = 1; k < 4; ++k) {
-            q[k] = mask ? __ffs(mask) - 1 : q[k - 1];
-            mask &= mask - 1;
+        for (int k = 0; k < 4; ++k) {
+            int iy = qj - 1 + k, iz = qk - 1 + k;
+            if (k == 0) {
+                iy += iy < 0 ? ny : 0;
+                iz += iz < 0 ? nz : 0;
+            } else if (k > 1) {
+                iy -= iy >= ny ? ny : 0;
+                iz -= iz >= nz ? nz : 0;
+            }
+            oy[k] = ix + nx * iy;
+            oz[k] = nx * ny * iz;
+            wz[k] = cubic_w(cubic_coef(k), fz);
         }
-        float sk[4][6];
+        const float wx = cubic_w(cx, fx);
+        float s0[6], s1[6], v[6];
+        cubic_rows(tab, oy[0], oz, wx * cubic_w(cubic_coef(0), fy), wz, s0);
+        cubic_rows(tab, oy[2], oz, wx * cubic_w(cubic_coef(2), fy), wz, s1);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            cubic_share(g, tab, __shfl_sync(full, ci[0], q[k]), __shfl_sync(full, ci[1], q[k]),
-                        __shfl_sync(full, ci[2], q[k]), __shfl_sync(full, cf[0], q[k]),
-                        __shfl_sync(full, cf[1], q[k]), __shfl_sync(full, cf[2], q[k]), sk[k]);
-        float r[3];
-        reduce4x6(sk, r);
-        // the owner of particle k takes E from lane (k >> 1) << 4 | (k & 1) << 3
-        // and B from that lane + 4
-        int mine = -1;
+        for (int c = 0; c < 6; ++c) v[c] = __fadd_rn(s0[c], s1[c]);
+        cubic_rows(tab, oy[1], oz, wx * cubic_w(cubic_coef(1), fy), wz, s0);
+        cubic_rows(tab, oy[3], oz, wx * cubic_w(cubic_coef(3), fy), wz, s1);
 #pragma unroll
-        for (int k = 3; k >= 0; --k)
-            if (lane == q[k]) mine = k;
-        const int src = mine < 0 ? 0 : (((mine >> 1) << 4) | ((mine & 1) << 3));
-        const float ex = __shfl_sync(full, r[0], src), ey = __shfl_sync(full, r[1], src),
-                    ez = __shfl_sync(full, r[2], src);
-        const float bx = __shfl_sync(full, r[0], src + 4), by = __shfl_sync(full, r[1], src + 4),
-                    bz = __shfl_sync(full, r[2], src + 4);
-        if (mine >= 0) {
-            E = {ex, ey, ez};
-            B = {bx, by, bz};
+        for (int c = 0; c < 6; ++c) {
+            v[c] = __fadd_rn(v[c], __fadd_rn(s0[c], s1[c]));
+            v[c] += __shfl_xor_sync(full, v[c], 2);
+            v[c] += __shfl_xor_sync(full, v[c], 1);
+        }
+        if (want && d == r) {
+            E = {v[0], v[1], v[2]};
+            B = {v[3], v[4], v[5]};
         }
     }
 }
@@ -538,8 +489,10 @@ __device__ __forceinline__ void save_row32(const BorisArgs& a, int W, int64_t i,
     }
 }
 
+// four blocks per SM (128 registers, no spills in the loop): 4.68 ms on the first
+// ensemble above, five blocks 5.61, six 5.00 (7.81 against 6.10 on the second)
 template <bool MULTI>
-__global__ void __launch_bounds__(128, 5) k_cubic32c(BorisArgs a) {
+__global__ void __launch_bounds__(128, 4) k_cubic32c(BorisArgs a) {
     const int W = 6 + (a.save_fields ? 6 : 0) + (a.save_work ? 4 : 0);
     const uint64_t t_start = globaltimer_ns();
     const int64_t i = take_particle(a, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
