@@ -13,20 +13,10 @@
 
 namespace tpb {
 
-// the contraction of |t|^2 (dot_fma) in the steps, in the first half step and in the
+// the contraction of |t|^2 (dot_fma) in the steps, and in the first half step and the
 // saves, as k_fixed32c had it: a float rounding that differs in a step or at the
 // start grows 1000-fold in 250 steps of the turbulent field
 constexpr int kStep = 1, kSave = 2;
-template <bool MULTI>
-constexpr int kFirst = MULTI ? 1 : 2;
-
-// one update of length dt at (p, v) by the lane alone
-template <bool MULTI>
-__device__ __forceinline__ CV kick_grid32(const BorisArgs& a, CPos p, CV v, double dt) {
-    F3 E, B;
-    eval_EB32<true>(a.f, p, 0.0, E, B);
-    return vel32<MULTI, kFirst<MULTI>>(v, E, B, a, dt);
-}
 
 template <bool MULTI, bool PERIODIC>
 struct GridPush32 {
@@ -53,18 +43,18 @@ struct GridPush32 {
         dth = (float)dt;
         dtl = (float)(dt - (double)dth);
     }
+    static __device__ __forceinline__ bool axes(const DevField& g, const CPos& p, AxF& ax, AxF& ay, AxF& az) {
+        if (!PERIODIC) return axes32(g, p, ax, ay, az);
+        axis32_periodic(g, 0, p.hi[0], p.lo[0], ax);
+        axis32_periodic(g, 1, p.hi[1], p.lo[1], ay);
+        axis32_periodic(g, 2, p.hi[2], p.lo[2], az);
+        return true;
+    }
     // eval_EB32 with the stencils of the warp gathered by pairs of lanes
     static __device__ __forceinline__ F gather(const BorisArgs& a, const CPos& p) {
         const DevField& g = a.f.B;
         AxF ax, ay, az;
-        bool ok = true;
-        if (PERIODIC) {
-            axis32_periodic(g, 0, p.hi[0], p.lo[0], ax);
-            axis32_periodic(g, 1, p.hi[1], p.lo[1], ay);
-            axis32_periodic(g, 2, p.hi[2], p.lo[2], az);
-        } else {
-            ok = axes32(g, p, ax, ay, az);
-        }
+        const bool ok = axes(g, p, ax, ay, az);
         float c0[6], c1[6];
         pair_planes<float>(a.f.eb32, ok ? eb_node(g, ax.i0, ay.i0, az.i0) : 0, ok ? (ax.i1 - ax.i0) * g.n[1] * g.n[2] : 0,
                            ok ? (ay.i1 - ay.i0) * g.n[2] : 0, ok ? az.i1 - az.i0 : 0, ax.f, ay.f, c0, c1);
@@ -81,8 +71,12 @@ struct GridPush32 {
     __device__ __forceinline__ CV half(const BorisArgs& a, const CPos&, const CV& v, const F& f, double dt) const {
         return vel32<MULTI, kSave>(v, f.E, f.B, a, 0.5 * dt);
     }
+    // one update of length dt at (p, v) by the lane alone
     static __device__ __forceinline__ CV general(const BorisArgs& a, const CPos& p, const CV& v, double dt) {
-        return kick_grid32<MULTI>(a, p, v, dt);
+        AxF ax, ay, az;
+        F3 E = nanf3(), B = nanf3();
+        if (axes(a.f.B, p, ax, ay, az)) eb_gather32(a.f, ax, ay, az, E, B);
+        return vel32<MULTI, kSave>(v, E, B, a, dt);
     }
     __device__ __forceinline__ CPos advance(const BorisArgs& a, CPos p, const CV& v, double) const {
         cpos_push_cv(a, p, v, dth, dtl);

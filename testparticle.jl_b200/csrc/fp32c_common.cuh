@@ -287,6 +287,30 @@ __device__ __forceinline__ F3 analytic_eval32(const DevField& f, const CPos& p, 
     }
 }
 
+// E and B at a stencil of the interleaved table
+__device__ __forceinline__ void eb_gather32(const DevFields& F, const AxF& ax, const AxF& ay, const AxF& az, F3& E,
+                                            F3& B) {
+    const float4* T = F.eb32;
+    // 8 corners, each one aligned 32-byte sector (E xyz0, B xyz0) read by
+    // one 256-bit load; all issued before any use
+    float4 e000, b000, e100, b100, e010, b010, e110, b110;
+    float4 e001, b001, e101, b101, e011, b011, e111, b111;
+#define TPB_CORNER(X, Y, Z) ldg_node8(T + 2 * (int64_t)eb_node(F.B, ax.i##X, ay.i##Y, az.i##Z), e##X##Y##Z, b##X##Y##Z);
+    TPB_CORNER(0, 0, 0)
+    TPB_CORNER(1, 0, 0)
+    TPB_CORNER(0, 1, 0)
+    TPB_CORNER(1, 1, 0)
+    TPB_CORNER(0, 0, 1)
+    TPB_CORNER(1, 0, 1)
+    TPB_CORNER(0, 1, 1)
+    TPB_CORNER(1, 1, 1)
+#undef TPB_CORNER
+    E = tri3(xyz(e000), xyz(e100), xyz(e010), xyz(e110), xyz(e001), xyz(e101), xyz(e011),
+             xyz(e111), ax, ay, az);
+    B = tri3(xyz(b000), xyz(b100), xyz(b010), xyz(b110), xyz(b001), xyz(b101), xyz(b011),
+             xyz(b111), ax, ay, az);
+}
+
 template <bool PACKED_ONLY = false>
 __device__ __forceinline__ void eval_EB32(const DevFields& F, const CPos& p, double t, F3& E, F3& B) {
     if (PACKED_ONLY || F.eb32) {
@@ -296,25 +320,7 @@ __device__ __forceinline__ void eval_EB32(const DevFields& F, const CPos& p, dou
             B = E;
             return;
         }
-        const float4* T = F.eb32;
-        // 8 corners, each one aligned 32-byte sector (E xyz0, B xyz0) read by
-        // one 256-bit load; all issued before any use
-        float4 e000, b000, e100, b100, e010, b010, e110, b110;
-        float4 e001, b001, e101, b101, e011, b011, e111, b111;
-#define TPB_CORNER(X, Y, Z) ldg_node8(T + 2 * (int64_t)eb_node(F.B, ax.i##X, ay.i##Y, az.i##Z), e##X##Y##Z, b##X##Y##Z);
-        TPB_CORNER(0, 0, 0)
-        TPB_CORNER(1, 0, 0)
-        TPB_CORNER(0, 1, 0)
-        TPB_CORNER(1, 1, 0)
-        TPB_CORNER(0, 0, 1)
-        TPB_CORNER(1, 0, 1)
-        TPB_CORNER(0, 1, 1)
-        TPB_CORNER(1, 1, 1)
-#undef TPB_CORNER
-        E = tri3(xyz(e000), xyz(e100), xyz(e010), xyz(e110), xyz(e001), xyz(e101), xyz(e011),
-                 xyz(e111), ax, ay, az);
-        B = tri3(xyz(b000), xyz(b100), xyz(b010), xyz(b110), xyz(b001), xyz(b101), xyz(b011),
-                 xyz(b111), ax, ay, az);
+        eb_gather32(F, ax, ay, az, E, B);
         return;
     }
     E = (F.E.kind == TP_FIELD_GRID) ? grid_eval32(F.E, p)
