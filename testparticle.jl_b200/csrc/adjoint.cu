@@ -380,10 +380,12 @@ struct GridKeep {
 __device__ __forceinline__ F3 grid_eval_keep(const DevField& g, const CPos& p, GridKeep& k) {
     k.ok = axes32(g, p, k.ax, k.ay, k.az);
     if (!k.ok) return nanf3_();
-    tri_nodes(g, k.ax, k.ay, k.az, k.nd);
+    tri_nodes(g, k.ax, k.ay, k.az, k.nd);  // the gradient table has x fastest, the field's z
+    int zf[8];
+    tri_nodes_eb(g, k.ax, k.ay, k.az, zf);
     float4 q[8];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) q[c] = __ldg(g.tab32 + k.nd[c]);
+    for (int c = 0; c < 8; ++c) q[c] = __ldg(g.tab32 + zf[c]);
     F3 val;
     tri_val_jac(q, k.ax, k.ay, k.az, val, k.dx, k.dy, k.dz);
     return val;

@@ -440,6 +440,7 @@ static const void* select_kernel64(const BorisArgs& a, bool queue) {
     if (seg_config(a)) return seg_kernel64(a, queue);
     if (field_config_of(a.f) == FK_EBGRID && (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP))
         return grid_kernel64(a, queue);
+    if (gridb_config(a)) return gridb_kernel64(a, queue);
     const bool multi = a.alg == TP_ALG_MULTISTEP || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     if (multi) return queue ? pick_fk64<true, true>(adaptive, a) : pick_fk64<true, false>(adaptive, a);

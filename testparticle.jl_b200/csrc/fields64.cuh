@@ -56,11 +56,12 @@ __device__ __forceinline__ bool grid_axis(const DevField& g, int a, double x, Ax
     } else if (!(u >= 0.0 && u <= umax)) {
         return false;
     }
-    double fl = floor(u);
-    long long i = (long long)fl;
+    // 0 <= u <= na - 1 here, or NaN
+    int32_t i = (int32_t)u;
     if (i > na - 2) i = na - 2;
-    o.i0 = (int32_t)i;
-    o.i1 = o.i0 + 1;
+    if (i < 0) i = 0;
+    o.i0 = i;
+    o.i1 = i + 1;
     o.f = u - (double)i;
     return true;
 }
@@ -87,33 +88,35 @@ __device__ __forceinline__ void grid_axis_periodic(const DevField& g, int a, dou
     o.i1 = (i + 1 == na) ? 0 : i + 1;
 }
 
+// one 32-byte, 32-byte-aligned record in a single read-only load
+__device__ __forceinline__ void ldg_doubles4(const double* p, double w[4]) {
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(w[0]), "=d"(w[1]), "=d"(w[2]), "=d"(w[3]) : "l"(p));
+}
+
 __device__ __forceinline__ double lerp64(double a, double b, double f) { return a + f * (b - a); }
 
-// Load node `node` of a table with `stride` 4-vectors per node, at offset `off`.
+// Load a node of a table: one 256-bit load of a float64 record
 __device__ __forceinline__ D3 load_node(const void* tab, bool f64, int64_t idx) {
     if (f64) {
-        const double2* p = reinterpret_cast<const double2*>(tab) + 2 * idx;
-        double2 a = __ldg(p), b = __ldg(p + 1);
-        return {a.x, a.y, b.x};
+        double w[4];
+        ldg_doubles4(reinterpret_cast<const double*>(tab) + 4 * idx, w);
+        return {w[0], w[1], w[2]};
     }
     float4 q = __ldg(reinterpret_cast<const float4*>(tab) + idx);
     return {(double)q.x, (double)q.y, (double)q.z};
 }
 
-// Trilinear interpolation from precomputed axes; `stride`/`off` select a
-// field inside an interleaved table.
-__device__ __forceinline__ D3 tri64(const DevField& g, const void* tab, bool f64, int stride,
-                                    int off, const Ax& ax, const Ax& ay, const Ax& az) {
-    const int64_t nx = g.n[0], nxy = (int64_t)g.n[0] * g.n[1];
-    int64_t j0 = ay.i0 * nx, j1 = ay.i1 * nx, k0 = az.i0 * nxy, k1 = az.i1 * nxy;
-    D3 v000 = load_node(tab, f64, (ax.i0 + j0 + k0) * stride + off);
-    D3 v100 = load_node(tab, f64, (ax.i1 + j0 + k0) * stride + off);
-    D3 v010 = load_node(tab, f64, (ax.i0 + j1 + k0) * stride + off);
-    D3 v110 = load_node(tab, f64, (ax.i1 + j1 + k0) * stride + off);
-    D3 v001 = load_node(tab, f64, (ax.i0 + j0 + k1) * stride + off);
-    D3 v101 = load_node(tab, f64, (ax.i1 + j0 + k1) * stride + off);
-    D3 v011 = load_node(tab, f64, (ax.i0 + j1 + k1) * stride + off);
-    D3 v111 = load_node(tab, f64, (ax.i1 + j1 + k1) * stride + off);
+// Trilinear interpolation of a grid's node table from precomputed axes
+__device__ __forceinline__ D3 tri64(const DevField& g, const Ax& ax, const Ax& ay, const Ax& az) {
+    const bool f64 = g.f64 != 0;
+    D3 v000 = load_node(g.tab, f64, tri_node(g, ax.i0, ay.i0, az.i0));
+    D3 v100 = load_node(g.tab, f64, tri_node(g, ax.i1, ay.i0, az.i0));
+    D3 v010 = load_node(g.tab, f64, tri_node(g, ax.i0, ay.i1, az.i0));
+    D3 v110 = load_node(g.tab, f64, tri_node(g, ax.i1, ay.i1, az.i0));
+    D3 v001 = load_node(g.tab, f64, tri_node(g, ax.i0, ay.i0, az.i1));
+    D3 v101 = load_node(g.tab, f64, tri_node(g, ax.i1, ay.i0, az.i1));
+    D3 v011 = load_node(g.tab, f64, tri_node(g, ax.i0, ay.i1, az.i1));
+    D3 v111 = load_node(g.tab, f64, tri_node(g, ax.i1, ay.i1, az.i1));
     D3 o;
 #define TPB_TRI(c)                                              \
     {                                                           \
@@ -170,7 +173,7 @@ __device__ __forceinline__ D3 grid_eval64(const DevField& g, D3 r) {
     if (GEN && g.general) return grid_general64(*g.self, r);
     Ax ax, ay, az;
     if (!grid_axes64(g, r, ax, ay, az)) return nan3();
-    return tri64(g, g.tab, g.f64 != 0, 1, 0, ax, ay, az);
+    return tri64(g, ax, ay, az);
 }
 
 // Analytic fields: ZERO, UNIFORM, AFFINE, DIPOLE (order of the oracle).
@@ -593,7 +596,7 @@ __device__ __forceinline__ void field_jac64(const DevField& f, D3 r, double t, D
                 for (int k = 0; k < 9; ++k) J[k] = F.x;
                 return;
             }
-            F = tri64(f, f.tab, f.f64 != 0, 1, 0, ax, ay, az);
+            F = tri64(f, ax, ay, az);
             double sx = f.inv_dx[0], sy = f.inv_dx[1], sz = f.inv_dx[2];
             if (f.bc == TP_BC_CLAMP) {
                 double ux = (r.x - f.x0[0]) * f.inv_dx[0], uy = (r.y - f.x0[1]) * f.inv_dx[1],
@@ -602,13 +605,15 @@ __device__ __forceinline__ void field_jac64(const DevField& f, D3 r, double t, D
                 if (uy < 0.0 || uy > (double)(f.n[1] - 1)) sy = 0.0;
                 if (uz < 0.0 || uz > (double)(f.n[2] - 1)) sz = 0.0;
             }
-            const int64_t nx = f.n[0], nxy = (int64_t)f.n[0] * f.n[1];
-            int64_t j0 = ay.i0 * nx, j1 = ay.i1 * nx, k0 = az.i0 * nxy, k1 = az.i1 * nxy;
-            bool f64 = f.f64 != 0;
-            D3 w000 = load_node(f.tab, f64, ax.i0 + j0 + k0), w100 = load_node(f.tab, f64, ax.i1 + j0 + k0);
-            D3 w010 = load_node(f.tab, f64, ax.i0 + j1 + k0), w110 = load_node(f.tab, f64, ax.i1 + j1 + k0);
-            D3 w001 = load_node(f.tab, f64, ax.i0 + j0 + k1), w101 = load_node(f.tab, f64, ax.i1 + j0 + k1);
-            D3 w011 = load_node(f.tab, f64, ax.i0 + j1 + k1), w111 = load_node(f.tab, f64, ax.i1 + j1 + k1);
+            const bool f64 = f.f64 != 0;
+            D3 w000 = load_node(f.tab, f64, tri_node(f, ax.i0, ay.i0, az.i0));
+            D3 w100 = load_node(f.tab, f64, tri_node(f, ax.i1, ay.i0, az.i0));
+            D3 w010 = load_node(f.tab, f64, tri_node(f, ax.i0, ay.i1, az.i0));
+            D3 w110 = load_node(f.tab, f64, tri_node(f, ax.i1, ay.i1, az.i0));
+            D3 w001 = load_node(f.tab, f64, tri_node(f, ax.i0, ay.i0, az.i1));
+            D3 w101 = load_node(f.tab, f64, tri_node(f, ax.i1, ay.i0, az.i1));
+            D3 w011 = load_node(f.tab, f64, tri_node(f, ax.i0, ay.i1, az.i1));
+            D3 w111 = load_node(f.tab, f64, tri_node(f, ax.i1, ay.i1, az.i1));
             double fx = ax.f, fy = ay.f, fz = az.f;
 #define TPB_GJ(c, row)                                                                  \
     {                                                                                   \

@@ -251,12 +251,10 @@ __device__ __forceinline__ F3 grid_eval32(const DevField& g, const CPos& p) {
     AxF ax, ay, az;
     if (!axes32(g, p, ax, ay, az)) return nanf3();
     const float4* T = g.tab32;
-    const int nx = g.n[0], nxy = g.n[0] * g.n[1];
-    int j0 = ay.i0 * nx, j1 = ay.i1 * nx, k0 = az.i0 * nxy, k1 = az.i1 * nxy;
-    F3 v000 = xyz(__ldg(T + ax.i0 + j0 + k0)), v100 = xyz(__ldg(T + ax.i1 + j0 + k0));
-    F3 v010 = xyz(__ldg(T + ax.i0 + j1 + k0)), v110 = xyz(__ldg(T + ax.i1 + j1 + k0));
-    F3 v001 = xyz(__ldg(T + ax.i0 + j0 + k1)), v101 = xyz(__ldg(T + ax.i1 + j0 + k1));
-    F3 v011 = xyz(__ldg(T + ax.i0 + j1 + k1)), v111 = xyz(__ldg(T + ax.i1 + j1 + k1));
+    F3 v000 = xyz(__ldg(T + eb_node(g, ax.i0, ay.i0, az.i0))), v100 = xyz(__ldg(T + eb_node(g, ax.i1, ay.i0, az.i0)));
+    F3 v010 = xyz(__ldg(T + eb_node(g, ax.i0, ay.i1, az.i0))), v110 = xyz(__ldg(T + eb_node(g, ax.i1, ay.i1, az.i0)));
+    F3 v001 = xyz(__ldg(T + eb_node(g, ax.i0, ay.i0, az.i1))), v101 = xyz(__ldg(T + eb_node(g, ax.i1, ay.i0, az.i1)));
+    F3 v011 = xyz(__ldg(T + eb_node(g, ax.i0, ay.i1, az.i1))), v111 = xyz(__ldg(T + eb_node(g, ax.i1, ay.i1, az.i1)));
     return tri3(v000, v100, v010, v110, v001, v101, v011, v111, ax, ay, az);
 }
 

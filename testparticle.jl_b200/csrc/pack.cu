@@ -72,6 +72,42 @@ cudaError_t launch_pack_eb(const void* E, const void* B, int src_f64, const int3
     return cudaGetLastError();
 }
 
+// the data of one grid into its own node table, z fastest (tri_node)
+template <class S, class D>
+__global__ void __launch_bounds__(256) k_pack_tri(const S* src, int nx, int ny, int nz, D* dst) {
+    __shared__ D tile[3][32][33];
+    const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32, lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    for (int y = blockIdx.z; y < ny; y += gridDim.z) {
+        for (int r = row; r < 32; r += 8)
+            if (z0 + r < nz) {
+                const int64_t k = 3 * (x0 + (int64_t)nx * (y + (int64_t)ny * (z0 + r)));
+                const int m = 3 * (nx - x0 < 32 ? nx - x0 : 32);
+                for (int j = lane; j < m; j += 32) tile[j % 3][r][j / 3] = (D)src[k + j];
+            }
+        __syncthreads();
+        for (int r = row; r < 32; r += 8)
+            if (x0 + r < nx && z0 + lane < nz) {
+                D* o = dst + 4 * (z0 + lane + (int64_t)nz * (y + (int64_t)ny * (x0 + r)));
+                o[0] = tile[0][lane][r];
+                o[1] = tile[1][lane][r];
+                o[2] = tile[2][lane][r];
+                o[3] = (D)0;
+            }
+        __syncthreads();
+    }
+}
+
+cudaError_t launch_pack_tri(const void* src, int src_f64, const int32_t n[3], void* dst, int dst_f64, cudaStream_t s) {
+    const dim3 grid((n[0] + 31) / 32, (n[2] + 31) / 32, n[1] < 65535 ? n[1] : 65535);
+    if (src_f64 && dst_f64)
+        k_pack_tri<double, double><<<grid, 256, 0, s>>>((const double*)src, n[0], n[1], n[2], (double*)dst);
+    else if (src_f64)
+        k_pack_tri<double, float><<<grid, 256, 0, s>>>((const double*)src, n[0], n[1], n[2], (float*)dst);
+    else
+        k_pack_tri<float, float><<<grid, 256, 0, s>>>((const float*)src, n[0], n[1], n[2], (float*)dst);
+    return cudaGetLastError();
+}
+
 // slot-major (t[k*n+i], u[(k*W+c)*n+i]) -> per-trajectory packed
 // (t_out[off_i + k], u_out[(off_i + k)*W + c]).  One warp per particle
 // group: threads stride over (particle, save) pairs.

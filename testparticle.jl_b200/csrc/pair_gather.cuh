@@ -1,7 +1,7 @@
 // pair_gather.cuh -- trilinear stencils gathered by pairs of lanes.
 //
-// A node of the interleaved table is 32 bytes (E xyz0, B xyz0), z is its fastest
-// axis, and a 128-byte line holds four nodes that are neighbours along z.  When
+// A node of the interleaved table (E xyz0, B xyz0) or of one float64 field is 32
+// bytes, z is the tables' fastest axis, and a 128-byte line holds four nodes that are neighbours along z.  When
 // every lane loads the 8 corners of its own particle, the 32 lanes of a load
 // instruction touch 32 different lines, and the L1 cache, which looks up one
 // line per clock, needs 8 x 32 clocks per warp and step: that bounded the
@@ -34,12 +34,48 @@ __device__ __forceinline__ void ldg_words8(const float4* p, float w[8]) {
         : "l"(p));
 }
 
-// E xyz, B xyz at the stencil's lower (c0) and upper (c1) z-plane, interpolated
-// along x and y.  `base` is the node of the lower corner, dx, dy, dz the node
-// offsets to the neighbours; fx, fy the fractions.
-template <class R>
-__device__ __forceinline__ void pair_planes(const float4* T, int base, int dx, int dy, int dz, R fx, R fy, R c0[6],
-                                            R c1[6]) {
+// node records: NC values of type W from the table at node `i`
+struct NodeEB {  // interleaved float table
+    static constexpr int NC = 6;
+    using W = float;
+    static __device__ __forceinline__ void load(const void* T, int i, W w[NC]) {
+        float r[8];
+        ldg_words8(static_cast<const float4*>(T) + 2 * (int64_t)i, r);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) w[c] = r[c < 3 ? c : c + 1];
+    }
+};
+struct Node32 {  // float table of one field
+    static constexpr int NC = 3;
+    using W = float;
+    static __device__ __forceinline__ void load(const void* T, int i, W w[NC]) {
+        const float4 q = __ldg(static_cast<const float4*>(T) + i);
+        w[0] = q.x;
+        w[1] = q.y;
+        w[2] = q.z;
+    }
+};
+struct Node64 {  // float64 table of one field
+    static constexpr int NC = 3;
+    using W = double;
+    static __device__ __forceinline__ void load(const void* T, int i, W w[NC]) {
+        double r[4];
+        asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+            : "=d"(r[0]), "=d"(r[1]), "=d"(r[2]), "=d"(r[3])
+            : "l"(static_cast<const double*>(T) + 4 * (int64_t)i));
+        w[0] = r[0];
+        w[1] = r[1];
+        w[2] = r[2];
+    }
+};
+
+// The node's values (E xyz, B xyz, or one field) at the stencil's lower (c0) and
+// upper (c1) z-plane, interpolated along x and y.  `base` is the node of the
+// lower corner, dx, dy, dz the node offsets to the neighbours; fx, fy the fractions.
+template <class R, class NODE = NodeEB>
+__device__ __forceinline__ void pair_planes(const void* T, int base, int dx, int dy, int dz, R fx, R fy, R c0[NODE::NC],
+                                            R c1[NODE::NC]) {
+    constexpr int NC = NODE::NC;
     const unsigned full = 0xffffffffu;
     const bool odd = threadIdx.x & 1;
     const int pb = __shfl_xor_sync(full, base + dz, 1);
@@ -48,22 +84,21 @@ __device__ __forceinline__ void pair_planes(const float4* T, int base, int dx, i
     // its lower plane, the partner its upper plane
     const int ab = odd ? pb : base, adx = odd ? pdx : dx, ady = odd ? pdy : dy;
     const int bb = odd ? base : pb, bdx = odd ? dx : pdx, bdy = odd ? dy : pdy;
-    float A[4][8], B[4][8];  // corners (x, y) = 00, 10, 01, 11
-    ldg_words8(T + 2 * (int64_t)ab, A[0]);
-    ldg_words8(T + 2 * (int64_t)(ab + adx), A[1]);
-    ldg_words8(T + 2 * (int64_t)(ab + ady), A[2]);
-    ldg_words8(T + 2 * (int64_t)(ab + adx + ady), A[3]);
-    ldg_words8(T + 2 * (int64_t)bb, B[0]);
-    ldg_words8(T + 2 * (int64_t)(bb + bdx), B[1]);
-    ldg_words8(T + 2 * (int64_t)(bb + bdy), B[2]);
-    ldg_words8(T + 2 * (int64_t)(bb + bdx + bdy), B[3]);
+    typename NODE::W A[4][NC], B[4][NC];  // corners (x, y) = 00, 10, 01, 11
+    NODE::load(T, ab, A[0]);
+    NODE::load(T, ab + adx, A[1]);
+    NODE::load(T, ab + ady, A[2]);
+    NODE::load(T, ab + adx + ady, A[3]);
+    NODE::load(T, bb, B[0]);
+    NODE::load(T, bb + bdx, B[1]);
+    NODE::load(T, bb + bdy, B[2]);
+    NODE::load(T, bb + bdx + bdy, B[3]);
     const R pfx = __shfl_xor_sync(full, fx, 1), pfy = __shfl_xor_sync(full, fy, 1);
     const R ax = odd ? pfx : fx, ay = odd ? pfy : fy, bx = odd ? fx : pfx, by = odd ? fy : pfy;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        const int k = c < 3 ? c : c + 1;
-        const R va = pair_lerp(pair_lerp((R)A[0][k], (R)A[1][k], ax), pair_lerp((R)A[2][k], (R)A[3][k], ax), ay);
-        const R vb = pair_lerp(pair_lerp((R)B[0][k], (R)B[1][k], bx), pair_lerp((R)B[2][k], (R)B[3][k], bx), by);
+    for (int c = 0; c < NC; ++c) {
+        const R va = pair_lerp(pair_lerp((R)A[0][c], (R)A[1][c], ax), pair_lerp((R)A[2][c], (R)A[3][c], ax), ay);
+        const R vb = pair_lerp(pair_lerp((R)B[0][c], (R)B[1][c], bx), pair_lerp((R)B[2][c], (R)B[3][c], bx), by);
         c0[c] = odd ? vb : va;
         c1[c] = __shfl_xor_sync(full, odd ? va : vb, 1);
     }

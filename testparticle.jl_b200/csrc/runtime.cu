@@ -604,6 +604,19 @@ DevTerm dev_term(const tp_term_desc& t) {
     return d;
 }
 
+// the node tables of a grid from its raw data: x fastest for the general
+// evaluators, z fastest (tri_node) for the trilinear ones
+cudaError_t pack_tables(tp_field* f, bool f64, bool general, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < (f64 ? 2 : 1) && e == cudaSuccess; ++k) {
+        void* dst = k == 0 ? f->d_tab : f->d_tab32;
+        const int dst64 = f64 && k == 0;
+        e = general ? launch_pack_node_table(f->d_raw, f64, f->nodes, dst, dst64, 1, 0, s)
+                    : launch_pack_tri(f->d_raw, f64, f->dev.n, dst, dst64, s);
+    }
+    return e;
+}
+
 // Build DevFields for a run; interleaves two grids on one geometry.
 int make_dev_fields(tp_ctx* ctx, const tp_field* E, tp_field* B, DevFields& F) {
     std::memset(&F, 0, sizeof(F));
@@ -934,13 +947,8 @@ int tp_field_create(tp_ctx* ctx, const tp_field_desc* d, tp_field** out) {
                 e = cudaMemcpyAsync(f->d_raw, d->data, (size_t)nodes * 3 * esz, cudaMemcpyDefault,
                                     ctx->stream);
             if (e == cudaSuccess) e = held_alloc(ctx, &f->d_tab, (size_t)nodes * 4 * esz);
-            if (e == cudaSuccess)
-                e = launch_pack_node_table(f->d_raw, f64, nodes, f->d_tab, f64, 1, 0, ctx->stream);
-            if (e == cudaSuccess && f64) {
-                e = held_alloc(ctx, &f->d_tab32, (size_t)nodes * 4 * sizeof(float));
-                if (e == cudaSuccess)
-                    e = launch_pack_node_table(f->d_raw, 1, nodes, f->d_tab32, 0, 1, 0, ctx->stream);
-            }
+            if (e == cudaSuccess && f64) e = held_alloc(ctx, &f->d_tab32, (size_t)nodes * 4 * sizeof(float));
+            if (e == cudaSuccess) e = pack_tables(f, f64, general, ctx->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
             if (e != cudaSuccess) {
                 int r = cuda_fail(ctx, e, "grid upload");
@@ -983,9 +991,7 @@ int tp_field_update(tp_field* f, const void* data) {
     bool f64 = f->desc.dtype == TP_DTYPE_F64;
     size_t esz = f64 ? sizeof(double) : sizeof(float);
     cudaError_t e = cudaMemcpyAsync(f->d_raw, data, (size_t)f->nodes * 3 * esz, cudaMemcpyDefault, ctx->stream);
-    if (e == cudaSuccess) e = launch_pack_node_table(f->d_raw, f64, f->nodes, f->d_tab, f64, 1, 0, ctx->stream);
-    if (e == cudaSuccess && f64)
-        e = launch_pack_node_table(f->d_raw, 1, f->nodes, f->d_tab32, 0, 1, 0, ctx->stream);
+    if (e == cudaSuccess) e = pack_tables(f, f64, f->dev.general != 0, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "grid update");
     // new identity: interleaved tables built with the old values are rebuilt

@@ -48,7 +48,7 @@ struct DevField {
     float coeff;
     float mhatf[3];   // dipole: unit moment and K = coef * |m| (keeps float
     float Kf;         //   intermediates normal: coef / r^5 alone underflows)
-    const void* tab;  // per-node table: float4 / double4 per node (x,y,z,0)
+    const void* tab;  // per-node table: float4 / double4 per node (x,y,z,0); tri_node, or x fastest (general)
     const float4* tab32;  // float table for the FP32C kernels (same as tab for float data)
     // grids off the trilinear uniform Cartesian 3-D fast path (grid_general.cuh)
     int32_t general;  // 1: order, geometry, dimension or axes differ from the fast path
@@ -101,10 +101,14 @@ struct DevFields {
     const float4* ebc32;
 };
 
-// node index in the interleaved table: z fastest, so that the two nodes a
-// stencil takes along z share a 128-byte line (pair_gather.cuh)
+// node index in the tables of a trilinear uniform-Cartesian grid (tab and tab32
+// where `general` is 0, and the interleaved table): z fastest, so that the two
+// nodes a stencil takes along z share a 128-byte line (pair_gather.cuh)
 __host__ __device__ __forceinline__ int eb_node(const DevField& g, int ix, int iy, int iz) {
     return iz + g.n[2] * (iy + g.n[1] * ix);
+}
+__host__ __device__ __forceinline__ int64_t tri_node(const DevField& g, int ix, int iy, int iz) {
+    return iz + (int64_t)g.n[2] * (iy + (int64_t)g.n[1] * ix);
 }
 
 // Termination predicate (the reference's isoutside, as flags).
@@ -197,6 +201,13 @@ __host__ __forceinline__ bool seg_config(const BorisArgs& a) {
     const int fk = kernel_config_of(a.f);
     if (a.alg == TP_ALG_ADAPTIVE) return fk == FK_DIPOLE;
     return (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP) && (fk == FK_DIPOLE || fk == FK_UNIFORM) && a.ppt != 2;
+}
+
+// fixed steps, E zero and B on a trilinear uniform-Cartesian grid
+__host__ __forceinline__ bool gridb_config(const BorisArgs& a) {
+    const DevField& B = a.f.B;
+    return (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP) && a.f.E.kind == TP_FIELD_ZERO &&
+           B.kind == TP_FIELD_GRID && !B.general;
 }
 
 // particle i's outputs are final: publish them, then count the particle

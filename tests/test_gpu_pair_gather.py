@@ -101,3 +101,33 @@ def test_interleaved_table_of_a_large_odd_grid(tp, orc):
     prob = tp.TraceProblem(u0, (0.0, 1.0e-3), tp.prepare(E, B))
     sols, ref = _both(tp, orc, prob, tp.Boris(), dt=1.0e-3, save_fields=True, trajectories=101)
     assert _rel(sols.u_all, ref.u) <= 1e-13
+
+
+@pytest.mark.parametrize("n", [(2, 2, 2), (3, 5, 2), (33, 34, 65)])
+@pytest.mark.parametrize("bc", ["wrap", "clamp", "fill"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_grid_push_b_alone(tp, orc, n, bc, dtype):
+    """E zero and B on a grid, float64: the oracle's operation order in every order of the update; lanes that start
+    outside a filled grid or at NaN stay NaN."""
+    edge = {"wrap": tp.WrapExtrap(), "clamp": tp.ClampExtrap(), "fill": tp.FillExtrap()}[bc]
+    B = _grid(tp, n, edge, dtype, 6)[1]
+    count = 70
+    rng = np.random.RandomState(count)
+    size = np.array(n) - (0 if bc == "wrap" else 1)
+    u0 = np.concatenate([DX * size[:, None] * rng.uniform(0.4, 0.6, (3, count)), 20.0 * rng.normal(size=(3, count))])
+    u0[:3, 1] = 0.0                  # a node
+    u0[:3, 2] = -2.3 * DX * size     # outside
+    u0[2, 3] = np.nan
+    if bc != "fill":
+        u0[3:, 4:] *= 1.0e4
+        u0[:3, 5] = DX * (size - 1)
+    steps = 40 - np.arange(count) % 3
+    dt = 2 * math.pi / (tp.qi / tp.mi * 5.0e-9) / 100
+    prob = tp.TraceProblem(u0, (0.0, 40 * dt), tp.prepare(tp.ZeroField(), B))
+    for alg in (tp.Boris(), tp.MultistepBoris2(), tp.MultistepBoris4(2), tp.MultistepBoris6(3)):
+        for ssi in (1, 17):
+            sols, ref = _both(tp, orc, prob, alg, dt=dt, tend=steps * dt, savestepinterval=ssi, trajectories=count)
+            _check_same_layout(sols, ref)
+            assert np.array_equal(sols.t_all, ref.t)
+            assert np.array_equal(np.isnan(sols.u_all), np.isnan(ref.u))
+            assert _rel(np.nan_to_num(sols.u_all), np.nan_to_num(ref.u)) <= 1e-13
