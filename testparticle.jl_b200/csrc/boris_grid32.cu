@@ -8,7 +8,6 @@
 // is the L1 cache (88 % busy): 5 line look-ups per particle and step, 11 shuffles
 // per warp, and the 8 sectors that come from L2.
 #include "boris32_common.cuh"
-#include "pair_gather.cuh"
 #include "seg_common.cuh"
 
 namespace tpb {
@@ -43,25 +42,9 @@ struct GridPush32 {
         dth = (float)dt;
         dtl = (float)(dt - (double)dth);
     }
-    static __device__ __forceinline__ bool axes(const DevField& g, const CPos& p, AxF& ax, AxF& ay, AxF& az) {
-        if (!PERIODIC) return axes32(g, p, ax, ay, az);
-        axis32_periodic(g, 0, p.hi[0], p.lo[0], ax);
-        axis32_periodic(g, 1, p.hi[1], p.lo[1], ay);
-        axis32_periodic(g, 2, p.hi[2], p.lo[2], az);
-        return true;
-    }
-    // eval_EB32 with the stencils of the warp gathered by pairs of lanes
     static __device__ __forceinline__ F gather(const BorisArgs& a, const CPos& p) {
-        const DevField& g = a.f.B;
-        AxF ax, ay, az;
-        const bool ok = axes(g, p, ax, ay, az);
-        float c0[6], c1[6];
-        pair_planes<float>(a.f.eb32, ok ? eb_node(g, ax.i0, ay.i0, az.i0) : 0, ok ? (ax.i1 - ax.i0) * g.n[1] * g.n[2] : 0,
-                           ok ? (ay.i1 - ay.i0) * g.n[2] : 0, ok ? az.i1 - az.i0 : 0, ax.f, ay.f, c0, c1);
         F f;
-        f.E = {lerp32(c0[0], c1[0], az.f), lerp32(c0[1], c1[1], az.f), lerp32(c0[2], c1[2], az.f)};
-        f.B = {lerp32(c0[3], c1[3], az.f), lerp32(c0[4], c1[4], az.f), lerp32(c0[5], c1[5], az.f)};
-        if (!ok) f.E = f.B = nanf3();
+        eb_pair_gather32<PERIODIC>(a.f, p, f.E, f.B);
         return f;
     }
     __device__ __forceinline__ bool kick(const BorisArgs& a, const CPos&, const CV& v, const F& f, CV& out) const {
@@ -75,7 +58,7 @@ struct GridPush32 {
     static __device__ __forceinline__ CV general(const BorisArgs& a, const CPos& p, const CV& v, double dt) {
         AxF ax, ay, az;
         F3 E = nanf3(), B = nanf3();
-        if (axes(a.f.B, p, ax, ay, az)) eb_gather32(a.f, ax, ay, az, E, B);
+        if (eb_axes32<PERIODIC>(a.f.B, p, ax, ay, az)) eb_gather32(a.f, ax, ay, az, E, B);
         return vel32<MULTI, kSave>(v, E, B, a, dt);
     }
     __device__ __forceinline__ CPos advance(const BorisArgs& a, CPos p, const CV& v, double) const {

@@ -7,6 +7,7 @@
 
 #include "fields64.cuh"
 #include "grid_general.cuh"
+#include "pair_gather.cuh"
 #include "tp_device.cuh"
 
 namespace tpb {
@@ -307,6 +308,32 @@ __device__ __forceinline__ void eb_gather32(const DevFields& F, const AxF& ax, c
              xyz(e111), ax, ay, az);
     B = tri3(xyz(b000), xyz(b100), xyz(b010), xyz(b110), xyz(b001), xyz(b101), xyz(b011),
              xyz(b111), ax, ay, az);
+}
+
+// the axes of a stencil in the interleaved table; false outside a grid that is
+// filled with NaN
+template <bool PERIODIC>
+__device__ __forceinline__ bool eb_axes32(const DevField& g, const CPos& p, AxF& ax, AxF& ay, AxF& az) {
+    if (!PERIODIC) return axes32(g, p, ax, ay, az);
+    axis32_periodic(g, 0, p.hi[0], p.lo[0], ax);
+    axis32_periodic(g, 1, p.hi[1], p.lo[1], ay);
+    axis32_periodic(g, 2, p.hi[2], p.lo[2], az);
+    return true;
+}
+
+// eval_EB32 with the stencils of the warp gathered by pairs of lanes: all 32
+// lanes call it together
+template <bool PERIODIC>
+__device__ __forceinline__ void eb_pair_gather32(const DevFields& F, const CPos& p, F3& E, F3& B) {
+    const DevField& g = F.B;
+    AxF ax, ay, az;
+    const bool ok = eb_axes32<PERIODIC>(g, p, ax, ay, az);
+    float c0[6], c1[6];
+    pair_planes<float>(F.eb32, ok ? eb_node(g, ax.i0, ay.i0, az.i0) : 0, ok ? (ax.i1 - ax.i0) * g.n[1] * g.n[2] : 0,
+                       ok ? (ay.i1 - ay.i0) * g.n[2] : 0, ok ? az.i1 - az.i0 : 0, ax.f, ay.f, c0, c1);
+    E = {lerp32(c0[0], c1[0], az.f), lerp32(c0[1], c1[1], az.f), lerp32(c0[2], c1[2], az.f)};
+    B = {lerp32(c0[3], c1[3], az.f), lerp32(c0[4], c1[4], az.f), lerp32(c0[5], c1[5], az.f)};
+    if (!ok) E = B = nanf3();
 }
 
 template <bool PACKED_ONLY = false>

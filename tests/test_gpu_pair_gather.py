@@ -131,3 +131,34 @@ def test_grid_push_b_alone(tp, orc, n, bc, dtype):
             assert np.array_equal(sols.t_all, ref.t)
             assert np.array_equal(np.isnan(sols.u_all), np.isnan(ref.u))
             assert _rel(np.nan_to_num(sols.u_all), np.nan_to_num(ref.u)) <= 1e-13
+
+
+@pytest.mark.parametrize("bc", ["wrap", "clamp", "fill"])
+@pytest.mark.parametrize("count", [1, 33, 150])
+def test_adjoint_forward(tp, bc, count):
+    """The recorded forward gathers as the FP32C push does: its final states stay within the same 40 x 2^-22 of the path."""
+    import torch
+    from testparticle_b200.autograd import GridTensor, boris_final_state
+
+    edge = {"wrap": tp.WrapExtrap(), "clamp": tp.ClampExtrap(), "fill": tp.FillExtrap()}[bc]
+    n = (7, 4, 9)
+    E, B = _grid(tp, n, edge, np.float32, 5)
+    rng = np.random.RandomState(count)
+    size = np.array(n) - 1
+    u0 = np.concatenate([DX * size[:, None] * rng.uniform(0.4, 0.6, (3, count)), 2.0e4 * rng.normal(size=(3, count))])
+    if bc != "fill" and count > 1:
+        u0[:3, 1] = -2.3 * DX * size
+    dt = 2 * math.pi / (tp.qi / tp.mi * 5.0e-9) / 100
+    E.data *= 0.1
+    want = tp.solve(tp.TraceProblem(u0, (0.0, 40 * dt), tp.prepare(E, B)), tp.Boris(), tp.EnsembleB200(precision="fp32c"),
+                    dt=dt, save_everystep=False, save_start=False, trajectories=count).u_all
+    grids = [GridTensor(torch.from_numpy(np.ascontiguousarray(f.data.T)).cuda().permute(3, 2, 1, 0), (0.0,) * 3, (DX,) * 3, edge)
+             for f in (E, B)]
+    got = boris_final_state(torch.from_numpy(np.ascontiguousarray(u0.T)).cuda(), *grids, q2m=tp.qi / tp.mi, dt=dt,
+                            tspan=(0.0, 40 * dt)).cpu().numpy()
+    path = 40 * dt * (np.linalg.norm(u0[3:], axis=0) + 1.0e5)
+    fine = np.isfinite(want).all(axis=1)  # a particle that leaves a filled grid ends in NaN
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    want, got, path = want[fine], got[fine], path[fine]
+    assert np.all(np.linalg.norm(got[:, :3] - want[:, :3], axis=1) <= 40 * 2.0**-22 * path)
+    assert np.all(np.linalg.norm(got[:, 3:] - want[:, 3:], axis=1) <= 40 * 2.0**-22 * path / (40 * dt))
