@@ -46,16 +46,16 @@ import __graft_entry__ as ge  # noqa: E402
 
 # gridded workload (config 2): algorithmic bytes of one particle-step, 8
 # trilinear corners x (E, B) x 3 float32, and the DRAM bytes per particle-step
-# of k_fixed32c measured by ncu (1.683 GB over 2e8 particle-steps; the 67 MB
-# field table is L2-resident)
+# measured by ncu for one thread per particle (1.683 GB over 2e8 particle-steps;
+# the 67 MB field table is L2-resident)
 BYTES_PER_PARTICLE_STEP = 192
 TRAFFIC_PER_PARTICLE_STEP = 8.4
 # dipole workload (config 3, MultistepBoris4(2)): algorithmic flops of one
 # particle-step (the rotation 121, the dipole 29), and the warp instructions
-# one warp-step of k_fixed32c<MULTI, queue, analytic> issues and the DRAM
-# bytes per particle-step, both measured by ncu on 262144 protons x 200 steps
+# one warp-step of the dipole's segment kernel issues and the DRAM bytes per
+# particle-step, both measured by ncu
 FLOPS_PER_PARTICLE_STEP_DIPOLE = 150
-INST_PER_WARP_STEP_DIPOLE = 340.8
+INST_PER_WARP_STEP_DIPOLE = 249.0
 TRAFFIC_PER_PARTICLE_STEP_DIPOLE = 0.32
 PEAKS_FILE = ROOT / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6650.0
@@ -661,14 +661,14 @@ def gridded_roofline(r, world, args, peak, peak_kind):
     kernel_s = r["tot32"] * 1e-3 / args.steps
     achieved = BYTES_PER_PARTICLE_STEP * r["ps_step"] / kernel_s / 1e9
     sm_clock = (r["clocks"].get("sm_mhz") or 1965.0) * 1e6
-    l1_ceiling = SMS * sm_clock / 8  # one L1 wavefront per SM clock, 8 corner lines per particle-step
+    l1_ceiling = SMS * sm_clock / 5  # one L1 line look-up per SM clock, 5 per particle-step (pairs of lanes share lines)
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": TRAFFIC_PER_PARTICLE_STEP * r["ps_step"],
             "note": f"{BYTES_PER_PARTICLE_STEP} algorithmic B/particle-step; peak {peak_kind}; the field table is "
                     f"L2-resident (DRAM {TRAFFIC_PER_PARTICLE_STEP} B/particle-step by ncu), so the binding "
                     "ceiling is the L1 wavefront one beside this"}
     l1 = {"value": l1_ceiling, "unit": "particle-steps/s", "frac": r["value"] / world / l1_ceiling,
-          "note": "148 SMs x SM clock / 8 corner lines per particle-step"}
+          "note": "148 SMs x SM clock / 5 line look-ups per particle-step"}
     return roof, l1
 
 
@@ -684,7 +684,7 @@ def dipole_roofline(r, world, args):
             "frac": achieved / peak, "traffic": TRAFFIC_PER_PARTICLE_STEP_DIPOLE * r["ps_step"],
             "flops": {"per_particle_step": FLOPS_PER_PARTICLE_STEP_DIPOLE,
                       "achieved_tflops": FLOPS_PER_PARTICLE_STEP_DIPOLE * r["ps_step"] / kernel_s / 1e12},
-            "note": f"{INST_PER_WARP_STEP_DIPOLE:.0f} warp instructions per warp-step (ncu, 262144 x 200 steps) x "
+            "note": f"{INST_PER_WARP_STEP_DIPOLE:.0f} warp instructions per warp-step (ncu) x "
                     "warp-steps / kernel time, against 148 SMs x 4 issue slots x the sampled SM clock; "
                     "MEASURED_PEAKS.json holds no FP32 or FP64 peak, so the flop rate is stated without a "
                     "fraction; DRAM traffic (inputs and saves only) by ncu"}

@@ -19,6 +19,8 @@
 //    of the cancellation the Taylor branch (multistep_boris.jl:99-108) guards;
 //  * time t, the adaptive step dt = C/|B| and the end-of-span clipping in
 //    float64 so that step decisions follow the float64 controller.
+// The dipole, uniform fields, and E and B on one trilinear grid have kernels of
+// their own (boris_seg32.cu, boris_grid32.cu); k_fixed32c takes the others.
 #include "boris32_common.cuh"
 
 namespace tpb {

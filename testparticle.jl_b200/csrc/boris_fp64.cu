@@ -14,10 +14,13 @@
 //
 // Kernels (MULTI: Multistep update; QUEUE: schedule; FK: field configuration,
 // see tp_device.cuh):
-//   k_fixed64<MULTI, QUEUE, FK, PPT>  _boris_single + _boris_loop!  (boris.jl:445-557)
+//   k_fixed64<MULTI, QUEUE, FK>    _boris_single + _boris_loop!  (boris.jl:445-557)
 //                                  with Boris (boris.jl:19-45) or
 //                                  Multistep (multistep_boris.jl:65-142) updates
 //   k_adaptive64<MULTI, QUEUE, FK> _adaptive_boris_single (adaptive_boris.jl:145-266)
+// The configurations with kernels of their own (a dipole or uniform fields, E and
+// B on one trilinear grid, B alone on one) run those of boris_seg64.cu and
+// boris_grid64.cu instead; k_fixed64 takes every other one.
 #include "boris64_common.cuh"
 
 namespace tpb {

@@ -254,15 +254,12 @@ __device__ __forceinline__ int64_t calc_nout(int64_t nt, int64_t ssi, bool ss, b
 
 }  // namespace tpb
 
-// Largest block a push kernel is compiled for, per field configuration: it
-// caps the register allocation at 65536 / TPB_MAXT(FK) per thread.  The
-// interleaved-grid kernels are gather-latency bound, so they take 384 (<= 170
-// registers: three 128-thread blocks per SM); at 512 the float64 one spills
-// 340 bytes per thread and measured 7 % slower on the 128^3 gridded
-// workload (1.93e10 against 2.07e10 particle-steps/s, four blocks per SM
-// instead of three), and the FP32C one spills 70-110 bytes and measured
-// 8 % slower at 448 or 512 (2.77e10 against 3.02e10): spills add traffic to
-// the L1 path that bounds it.  The analytic-field kernels are latency bound
+// Largest block a push launches with, per field configuration.  It also caps the
+// register allocation, at 65536 / TPB_MAXT(FK) per thread, of the kernels that
+// have no cap of their own (the segment kernels' is PUSH::kBound).  The
+// interleaved-grid ones still compiled with it (the adaptive pushes) are
+// gather-latency bound and take 384: at 512 they spill, which adds traffic to the
+// L1 path that bounds them.  The analytic-field kernels are latency bound
 // on float64 dependency chains and launch up to 512 threads: the float64
 // multistep and adaptive pushes in the dipole measured 15 % faster than at
 // 256 (the fixed-step and adaptive ones are compiled for larger blocks
@@ -274,10 +271,10 @@ __device__ __forceinline__ int64_t calc_nout(int64_t nt, int64_t ssi, bool ss, b
 // threads (<= 80 registers per thread, six 128-thread blocks per SM) although
 // launches stay at or below TPB_MAXT: the extra resident warps hide the
 // float64 dependency latency that bounds them, and outweigh the 40-150 bytes
-// of spills this costs.  On the dipole ensemble (MultistepBoris4(2), 1e6 x 1e4)
-// the FP32C push measured 7.50e10 -> 7.93e10 particle-steps/s (caps of 640,
-// 896 and 1024 threads: 7.69e10, 7.64e10, 7.58e10) and the float64 push
-// 2.71e10 -> 2.88e10 (640: 2.80e10).
+// of spills this costs.  On the dipole ensemble (MultistepBoris4(2), 1e6 x 1e4),
+// before the dipole had kernels of its own, the FP32C push measured 7.50e10 ->
+// 7.93e10 particle-steps/s (caps of 640, 896 and 1024 threads: 7.69e10, 7.64e10,
+// 7.58e10) and the float64 push 2.71e10 -> 2.88e10 (640: 2.80e10).
 #define TPB_FIXED_BOUND(FK) ((FK) == FK_ANALYTIC ? 768 : TPB_MAXT(FK))
 
 // The same for the adaptive kernels in analytic fields (AdaptiveBoris(0.1)
