@@ -20,7 +20,8 @@
 //  * time t, the adaptive step dt = C/|B| and the end-of-span clipping in
 //    float64 so that step decisions follow the float64 controller.
 // The dipole, uniform fields, and E and B on one trilinear grid have kernels of
-// their own (boris_seg32.cu, boris_grid32.cu); k_fixed32c takes the others.
+// their own (boris_seg32.cu, boris_grid32.cu); k_fixed32c takes the others, and small
+// gridded ensembles with frequent saves (ebgrid_seg_config).
 #include "boris32_common.cuh"
 
 namespace tpb {
@@ -753,8 +754,7 @@ static const void* kernel_ptr32(bool adaptive, int ppt) {
     if (adaptive) return (const void*)k_adaptive32c<MULTI, QUEUE, FK>;
     if constexpr (FK == FK_ANALYTIC)
         if (ppt == 2) return (const void*)k_fixed32c_slots<MULTI, QUEUE, FK, 2>;
-    if constexpr (FK == FK_EBGRID) return nullptr;  // grid_kernel32
-    else return (const void*)k_fixed32c<MULTI, QUEUE, FK>;
+    return (const void*)k_fixed32c<MULTI, QUEUE, FK>;
 }
 
 template <bool MULTI, bool QUEUE>
@@ -777,7 +777,7 @@ static const void* select_kernel32(const BorisArgs& a, bool queue) {
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     if (cubic_coop_kernel(a)) return multi ? (const void*)k_cubic32c<true> : (const void*)k_cubic32c<false>;
     if (seg_config(a)) return seg_kernel32(a, queue);
-    if (field_config_of(a.f) == FK_EBGRID && !adaptive) return grid_kernel32(a, queue);
+    if (ebgrid_seg_config(a, 16)) return grid_kernel32(a, queue);
     const int fk = field_config_of(a.f);
     const int ppt = a.ppt;
     if (multi) return queue ? pick_fk32<true, true>(adaptive, fk, ppt) : pick_fk32<true, false>(adaptive, fk, ppt);

@@ -20,7 +20,8 @@
 //   k_adaptive64<MULTI, QUEUE, FK> _adaptive_boris_single (adaptive_boris.jl:145-266)
 // The configurations with kernels of their own (a dipole or uniform fields, E and
 // B on one trilinear grid, B alone on one) run those of boris_seg64.cu and
-// boris_grid64.cu instead; k_fixed64 takes every other one.
+// boris_grid64.cu instead; k_fixed64 takes every other one, and small gridded ensembles
+// with frequent saves (ebgrid_seg_config).
 #include "boris64_common.cuh"
 
 namespace tpb {
@@ -426,8 +427,7 @@ static const void* kernel_ptr64(bool adaptive, int ppt) {
     if (adaptive) return (const void*)k_adaptive64<MULTI, QUEUE, FK>;
     if constexpr (FK == FK_ANALYTIC)
         if (ppt == 2) return (const void*)k_fixed64_slots<MULTI, QUEUE, FK, 2>;
-    if constexpr (FK == FK_EBGRID) return nullptr;  // grid_kernel64
-    else return (const void*)k_fixed64<MULTI, QUEUE, FK>;
+    return (const void*)k_fixed64<MULTI, QUEUE, FK>;
 }
 
 template <bool MULTI, bool QUEUE>
@@ -441,8 +441,7 @@ static const void* pick_fk64(bool adaptive, const BorisArgs& a) {
 
 static const void* select_kernel64(const BorisArgs& a, bool queue) {
     if (seg_config(a)) return seg_kernel64(a, queue);
-    if (field_config_of(a.f) == FK_EBGRID && (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP))
-        return grid_kernel64(a, queue);
+    if (ebgrid_seg_config(a, a.alg == TP_ALG_MULTISTEP ? 8 : 4)) return grid_kernel64(a, queue);
     if (gridb_config(a)) return gridb_kernel64(a, queue);
     const bool multi = a.alg == TP_ALG_MULTISTEP || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;

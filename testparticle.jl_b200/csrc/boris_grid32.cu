@@ -3,10 +3,8 @@
 // (pair_gather.cuh).  The arithmetic is that of Vel32<FK_EBGRID>.
 //
 // Measured on the 128^3 turbulent field, 1e6 protons, device time: 250 steps 8.43
-// -> 5.37 ms (4.7e10 particle-steps/s), 5.71 while the particles were still sorted by
-// cell first.  What bounds it
-// is the L1 cache (88 % busy): 5 line look-ups per particle and step, 11 shuffles
-// per warp, and the 8 sectors that come from L2.
+// -> 5.29 ms (4.7e10 particle-steps/s).  What bounds it is the L1 cache (88 % busy): 5 line
+// look-ups per particle and step, 11 shuffles per warp, and the 8 sectors that come from L2.
 #include "boris32_common.cuh"
 #include "seg_common.cuh"
 
@@ -28,7 +26,7 @@ struct GridPush32 {
     struct F {
         F3 E, B;
     };
-    static constexpr bool kWarp = true;
+    static constexpr bool kWarp = true, kJoin = MULTI;
     float h, dth, dtl;
     static __device__ __forceinline__ void init(const BorisArgs& a, CPos& p, CV& v, const double* u0) {
         cpos_init(a, p, u0);
@@ -51,16 +49,10 @@ struct GridPush32 {
         out = vel32h<MULTI, kStep>(v, f.E, f.B, a, h);
         return true;
     }
-    __device__ __forceinline__ CV half(const BorisArgs& a, const CPos&, const CV& v, const F& f, double dt) const {
-        return vel32<MULTI, kSave>(v, f.E, f.B, a, 0.5 * dt);
+    static __device__ __forceinline__ CV update(const BorisArgs& a, const CPos&, const CV& v, const F& f, double x, bool) {
+        return vel32<MULTI, kSave>(v, f.E, f.B, a, x);
     }
-    // one update of length dt at (p, v) by the lane alone
-    static __device__ __forceinline__ CV general(const BorisArgs& a, const CPos& p, const CV& v, double dt) {
-        AxF ax, ay, az;
-        F3 E = nanf3(), B = nanf3();
-        if (eb_axes32<PERIODIC>(a.f.B, p, ax, ay, az)) eb_gather32(a.f, ax, ay, az, E, B);
-        return vel32<MULTI, kSave>(v, E, B, a, dt);
-    }
+    static __device__ __forceinline__ CV refused(const BorisArgs&, const CPos&, const CV& v, const F&, double) { return v; }
     __device__ __forceinline__ CPos advance(const BorisArgs& a, CPos p, const CV& v, double) const {
         cpos_push_cv(a, p, v, dth, dtl);
         return p;
@@ -70,16 +62,20 @@ struct GridPush32 {
     }
 };
 
+// Without a predicate no state is kept for a rollback, which takes copies in every step:
+// 1e6 protons x 250 steps 5.95 -> 5.29 ms, with ends at different steps 2.85 -> 2.34 (400000
+// x 200; unrolling the loop twice instead: 5.41 and 3.38, instruction cache misses)
 template <bool MULTI, bool PERIODIC>
-static const void* grid_ptr32(bool queue) {
+static const void* grid_ptr32(bool queue, bool term) {
     using P = GridPush32<MULTI, PERIODIC>;
+    if (!queue && !term) return (const void*)k_seg<false, P, false>;
     return queue ? (const void*)k_seg<true, P> : (const void*)k_seg<false, P>;
 }
 
 const void* grid_kernel32(const BorisArgs& a, bool queue) {
-    const bool multi = a.alg == TP_ALG_MULTISTEP;
-    if (a.f.B.bc == TP_BC_PERIODIC) return multi ? grid_ptr32<true, true>(queue) : grid_ptr32<false, true>(queue);
-    return multi ? grid_ptr32<true, false>(queue) : grid_ptr32<false, false>(queue);
+    const bool multi = a.alg == TP_ALG_MULTISTEP, term = a.term.flags != 0;
+    if (a.f.B.bc == TP_BC_PERIODIC) return multi ? grid_ptr32<true, true>(queue, term) : grid_ptr32<false, true>(queue, term);
+    return multi ? grid_ptr32<true, false>(queue, term) : grid_ptr32<false, false>(queue, term);
 }
 
 }  // namespace tpb

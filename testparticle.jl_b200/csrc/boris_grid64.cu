@@ -41,7 +41,7 @@ struct GridPush64 {
     struct F {
         D3 E, B;
     };
-    static constexpr bool kWarp = true;
+    static constexpr bool kWarp = true, kJoin = MULTI;
     double h;
     static __device__ __forceinline__ void init(const BorisArgs&, D3& r, D3& v, const double* u0) {
         r = {u0[0], u0[1], u0[2]};
@@ -71,13 +71,11 @@ struct GridPush64 {
         out = multistep_rot64(v, f.E, f.B, a.q2m, h, a.order, a.nsub);
         return true;
     }
-    __device__ __forceinline__ D3 half(const BorisArgs& a, D3, D3 v, const F& f, double dt) const {
-        return vel_update64<MULTI>(v, f.E, f.B, a.q2m, 0.5 * dt, a.order, a.nsub);
+    static __device__ __forceinline__ D3 update(const BorisArgs& a, D3, D3 v, const F& f, double x, bool) {
+        return vel_update64<MULTI>(v, f.E, f.B, a.q2m, x, a.order, a.nsub);
     }
-    static __device__ __forceinline__ D3 general(const BorisArgs& a, D3 r, D3 v, double dt) {
-        D3 E, B;
-        eb_eval64_f32(a.f, r, E, B);
-        return vel_update64<MULTI>(v, E, B, a.q2m, dt, a.order, a.nsub);
+    static __device__ __forceinline__ D3 refused(const BorisArgs& a, D3 r, D3 v, const F& f, double dt) {
+        return update(a, r, v, f, dt, false);
     }
     static __device__ __forceinline__ D3 advance(const BorisArgs&, D3 r, D3 v, double dt) { return r + v * dt; }
     static __device__ __forceinline__ bool outside(const BorisArgs& a, D3 r, D3 v, double t) {
@@ -123,13 +121,15 @@ struct GridBPush64 : GridPush64<ORD != 0, PERIODIC> {
         return fast(a, v, f, h, out);
     }
     // half the factor is the factor of half the step, exactly
-    __device__ __forceinline__ D3 half(const BorisArgs& a, D3, D3 v, const F& f, double dt) const {
+    __device__ __forceinline__ D3 update(const BorisArgs& a, D3 r, D3 v, const F& f, double x, bool half) const {
         D3 out;
-        if (fast(a, v, f, 0.5 * h, out)) return out;
-        return vel_update64<MULTI>(v, {0.0, 0.0, 0.0}, f.B, a.q2m, 0.5 * dt, a.order, a.nsub);
+        double hh = 0.5 * h;
+        if (!half) hh = MULTI ? a.q2m * x / (double)(2 * a.nsub) : a.q2m * 0.5 * x;
+        if (fast(a, v, f, hh, out)) return out;
+        return refused(a, r, v, f, x);
     }
-    static __device__ __forceinline__ D3 general(const BorisArgs& a, D3 r, D3 v, double dt) {
-        return vel_update64<MULTI>(v, {0.0, 0.0, 0.0}, grid_eval64<false>(a.f.B, r), a.q2m, dt, a.order, a.nsub);
+    static __device__ __forceinline__ D3 refused(const BorisArgs& a, D3, D3 v, const F& f, double x) {
+        return vel_update64<MULTI>(v, {0.0, 0.0, 0.0}, f.B, a.q2m, x, a.order, a.nsub);
     }
 };
 

@@ -5,7 +5,7 @@
 // the field kind, the Multistep order and the absence of E known at compile time.
 //
 // Measured on the device against the general kernels, dipole, 1e6 protons x 1000
-// steps: MultistepBoris4(2) 12.44 -> 9.19 ms, Boris 10.93 -> 7.73 ms; 300001
+// steps: MultistepBoris4(2) 12.44 -> 9.03 ms, Boris 10.93 -> 7.73 ms; 300001
 // protons with AdaptiveBoris(0.1) of at most 1000 steps 4.81 -> 4.04 ms.  A
 // Multistep step is 249 warp instructions (341 before): 87 on the float64 pipe,
 // 73 FMA, 38 ALU, 23 XU (float <-> float64 conversions); issue is 70 % busy,
@@ -37,12 +37,11 @@ struct Push32 {
     static __device__ __forceinline__ D3 general(const BorisArgs& a, const CPos& p, D3 v, double dt) {
         return kick_general32<MULTI>(a, p, v, dt);
     }
+    template <class F>
+    static __device__ __forceinline__ D3 refused(const BorisArgs&, const CPos&, D3 v, const F&, double) { return v; }  // kick never refuses
     struct F {};
-    static constexpr bool kWarp = false;
+    static constexpr bool kWarp = false, kJoin = MULTI;
     static __device__ __forceinline__ F fields(const BorisArgs&, const CPos&) { return {}; }
-    __device__ __forceinline__ D3 half(const BorisArgs& a, const CPos& p, D3 v, F, double dt) const {
-        return kick_general32<MULTI>(a, p, v, 0.5 * dt);
-    }
     static __device__ __forceinline__ CPos advance(const BorisArgs& a, CPos p, D3 v, double dt) {
         cpos_push_d(a, p, v, dt);
         return p;
@@ -54,10 +53,10 @@ struct Push32 {
 
 template <bool MULTI, int ORD>
 struct DipolePush32 : Push32<MULTI> {
-    // register caps (threads), on the ensembles above.  Multistep: 512 10.0 ms,
-    // 640 9.65, 768 9.19, 1024 9.34; Boris: 512 8.67, 640 8.14, 768 8.05,
-    // 1024 7.73; adaptive: 512 4.06, 640 4.04, 768 4.38, 1024 4.30
-    static constexpr int kBound = MULTI ? 768 : 1024;
+    // register caps (threads), on the ensembles above.  Multistep: 640 9.55 ms, 768 9.30,
+    // 896 9.03, 1024 9.24; Boris: 512 8.67, 640 8.14, 768 8.05, 1024 7.73; adaptive:
+    // 512 4.06, 640 4.04, 768 4.38, 1024 4.30
+    static constexpr int kBound = MULTI ? 896 : 1024;
     static constexpr int kAdaptiveBound = 640;
     double h;
     __device__ __forceinline__ void start(const BorisArgs& a, double dt) {
@@ -73,8 +72,8 @@ struct DipolePush32 : Push32<MULTI> {
         return true;
     }
     // half the factor is the factor of half the step, exactly
-    __device__ __forceinline__ D3 half(const BorisArgs& a, const CPos&, D3 v, D3 B, double) const {
-        return rotate(a, v, B, 0.5 * h);
+    __device__ __forceinline__ D3 update(const BorisArgs& a, const CPos& p, D3 v, D3 B, double x, bool half) const {
+        return half ? rotate(a, v, B, 0.5 * h) : kick_general32<MULTI>(a, p, v, x);
     }
     // adaptive steps
     using Bv = D3;
@@ -101,6 +100,7 @@ struct DipolePush32 : Push32<MULTI> {
 // in uniform fields the rotation of a step depends on dt alone
 template <bool MULTI>
 struct UniformPush32 : Push32<MULTI> {
+    static constexpr bool kJoin = true;
     static constexpr int kBound = TPB_MAXT(FK_ANALYTIC);
     RotMixed m;
     __device__ __forceinline__ void start(const BorisArgs& a, double dt) {
@@ -113,6 +113,9 @@ struct UniformPush32 : Push32<MULTI> {
     __device__ __forceinline__ bool kick(const BorisArgs& a, const CPos&, D3 v, typename Push32<MULTI>::F, D3& out) const {
         out = rotate_mixed(v, m, a.f.E.kind != TP_FIELD_ZERO);
         return true;
+    }
+    static __device__ __forceinline__ D3 update(const BorisArgs& a, const CPos& p, D3 v, typename Push32<MULTI>::F, double x, bool) {
+        return kick_general32<MULTI>(a, p, v, x);
     }
 };
 

@@ -38,12 +38,13 @@ struct Push64 {
     static __device__ __forceinline__ D3 general(const BorisArgs& a, D3 r, D3 v, double dt) {
         return kick_general64<MULTI>(a, r, v, dt);
     }
-    struct F {};
-    static constexpr bool kWarp = false;
-    static __device__ __forceinline__ F fields(const BorisArgs&, D3) { return {}; }
-    __device__ __forceinline__ D3 half(const BorisArgs& a, D3 r, D3 v, F, double dt) const {
-        return kick_general64<MULTI>(a, r, v, 0.5 * dt);
+    template <class F>
+    static __device__ __forceinline__ D3 refused(const BorisArgs& a, D3 r, D3 v, const F&, double dt) {
+        return kick_general64<MULTI>(a, r, v, dt);
     }
+    struct F {};
+    static constexpr bool kWarp = false, kJoin = MULTI;
+    static __device__ __forceinline__ F fields(const BorisArgs&, D3) { return {}; }
     static __device__ __forceinline__ D3 advance(const BorisArgs&, D3 r, D3 v, double dt) { return r + v * dt; }
     static __device__ __forceinline__ bool outside(const BorisArgs& a, D3 r, D3 v, double t) {
         return outside64(a.term, r, v, t);
@@ -77,9 +78,11 @@ struct DipolePush64 : Push64<MULTI> {
         return fast(a, v, f, h, out);
     }
     // half the factor is the factor of half the step, exactly
-    __device__ __forceinline__ D3 half(const BorisArgs& a, D3 r, D3 v, const F& f, double dt) const {
+    __device__ __forceinline__ D3 update(const BorisArgs& a, D3 r, D3 v, const F& f, double x, bool half) const {
         D3 out;
-        return fast(a, v, f, 0.5 * h, out) ? out : kick_general64<MULTI>(a, r, v, 0.5 * dt);
+        double hh = 0.5 * h;
+        if (!half) hh = MULTI ? a.q2m * x / (double)(2 * a.nsub) : a.q2m * 0.5 * x;
+        return fast(a, v, f, hh, out) ? out : kick_general64<MULTI>(a, r, v, x);
     }
     // adaptive steps
     using Bv = D3;
@@ -124,8 +127,8 @@ struct UniformPush64<false> : Push64<false> {
         out = rotate(v, t, s, he);
         return true;
     }
-    __device__ __forceinline__ D3 half(const BorisArgs&, D3, D3 v, F, double) const {
-        return rotate(v, 0.5 * t, s2, 0.5 * he);
+    __device__ __forceinline__ D3 update(const BorisArgs& a, D3 r, D3 v, F, double x, bool half) const {
+        return half ? rotate(v, 0.5 * t, s2, 0.5 * he) : kick_general64<false>(a, r, v, x);
     }
     static __device__ __forceinline__ D3 rotate(D3 v, D3 t, D3 s, D3 he) {
         const D3 vm = v + he;
@@ -146,6 +149,9 @@ struct UniformPush64<true> : Push64<true> {
         e1 = m.c2 * m.e;
         e2 = m.c3 * cross(m.e, m.t);
         e3 = (m.c6 * dot(m.e, m.t)) * m.t;
+    }
+    static __device__ __forceinline__ D3 update(const BorisArgs& a, D3 r, D3 v, F, double x, bool) {
+        return kick_general64<true>(a, r, v, x);
     }
     __device__ __forceinline__ bool kick(const BorisArgs&, D3, D3 v, F, D3& out) const {
         out = m.c1 * v + m.c2 * cross(v, m.t);

@@ -593,17 +593,30 @@ __device__ __forceinline__ D3 cpos_d3(const CPos& p) {
             (double)p.hi[2] + (double)p.lo[2]};
 }
 
+// The contractions of this section are spelled out: a kernel that has the step in more
+// than one place (seg_common.cuh) must round it the same way in each, or an orbit
+// would depend on which lanes share its warp.
+__device__ __forceinline__ double dot_fma(D3 a, D3 b) { return fma(a.z, b.z, fma(a.x, b.x, __dmul_rn(a.y, b.y))); }
+__device__ __forceinline__ D3 cross_fma(D3 a, D3 b) {
+    return {fma(a.y, b.z, -__dmul_rn(a.z, b.y)), fma(a.z, b.x, -__dmul_rn(a.x, b.z)),
+            fma(a.x, b.y, -__dmul_rn(a.y, b.x))};
+}
+// s a + b
+__device__ __forceinline__ D3 axpy(double s, D3 a, D3 b) { return {fma(s, a.x, b.x), fma(s, a.y, b.y), fma(s, a.z, b.z)}; }
+__device__ __forceinline__ D3 scale_rn(double s, D3 a) { return {__dmul_rn(s, a.x), __dmul_rn(s, a.y), __dmul_rn(s, a.z)}; }
+
 __device__ __forceinline__ D3 dipole_mixed(const DevField& f, const CPos& p) {
     // B = coef (3 (m.d) d / r^5 - m / r^3), 1/r = y (1.5 - r^2 y^2 / 2)
     // from the float estimate y (relative error ~1e-13 after the step)
     const D3 d = cpos_d3(p) - D3{f.c[0], f.c[1], f.c[2]};
-    const double r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+    const double r2 = dot_fma(d, d);
     double y = (double)rsqrtf((float)r2);
-    y = y * fma(-0.5 * r2, y * y, 1.5);
-    const double ir2 = y * y;
-    const double k3 = f.coef * (ir2 * y);
-    const double k5 = 3.0 * (k3 * ir2) * (f.m[0] * d.x + f.m[1] * d.y + f.m[2] * d.z);
-    return {k5 * d.x - k3 * f.m[0], k5 * d.y - k3 * f.m[1], k5 * d.z - k3 * f.m[2]};
+    y = __dmul_rn(y, fma(-0.5 * r2, __dmul_rn(y, y), 1.5));
+    const double ir2 = __dmul_rn(y, y);
+    const double k3 = __dmul_rn(f.coef, __dmul_rn(ir2, y));
+    const double k5 = __dmul_rn(__dmul_rn(3.0, __dmul_rn(k3, ir2)), dot_fma(D3{f.m[0], f.m[1], f.m[2]}, d));
+    return {fma(k5, d.x, -__dmul_rn(k3, f.m[0])), fma(k5, d.y, -__dmul_rn(k3, f.m[1])),
+            fma(k5, d.z, -__dmul_rn(k3, f.m[2]))};
 }
 
 // analytic field in float64 at a compensated position
@@ -635,54 +648,56 @@ struct RotMixed {
 };
 
 __device__ __forceinline__ RotMixed rotation_mixed(D3 E, D3 B, double fac, int N, int n, bool hasE) {
-    D3 t = fac * B;
-    D3 e = hasE ? fac * E : D3{0.0, 0.0, 0.0};
-    double sd = dot(t, t);
+    D3 t = scale_rn(fac, B);
+    D3 e = hasE ? scale_rn(fac, E) : D3{0.0, 0.0, 0.0};
+    double sd = dot_fma(t, t);
     float s = (float)sd;
     if (N != 2) {
         float f_N, e_corr;
         if (N == 4) {
-            f_N = 1.0f + s * (1.0f / 3.0f);
+            f_N = fmaf(s, 1.0f / 3.0f, 1.0f);
             e_corr = -1.0f / 3.0f;
         } else {
-            f_N = 1.0f + s * (1.0f / 3.0f) + 2.0f * s * s * (1.0f / 15.0f);
-            e_corr = -1.0f / 3.0f - 2.0f * s * (1.0f / 15.0f);
+            const float s2 = __fmul_rn(2.0f, s);
+            f_N = fmaf(__fmul_rn(s2, s), 1.0f / 15.0f, fmaf(s, 1.0f / 3.0f, 1.0f));
+            e_corr = fmaf(-s2, 1.0f / 15.0f, -1.0f / 3.0f);
         }
         const double fd = f_N;
-        if (hasE) e = fd * e + ((double)e_corr * dot(e, t)) * t;
-        t = fd * t;
-        sd = (fd * fd) * sd;
+        if (hasE) e = axpy(__dmul_rn((double)e_corr, dot_fma(e, t)), t, scale_rn(fd, e));
+        t = scale_rn(fd, t);
+        sd = __dmul_rn(__dmul_rn(fd, fd), sd);
         s = (float)sd;
     }
-    float zr = 1.0f, q = 1.0f, A = 1.0f + s, R = 1.0f;  // after the first of the n >= 1 substeps
+    const float s1 = __fadd_rn(1.0f, s);
+    float zr = 1.0f, q = 1.0f, A = s1, R = 1.0f;  // after the first of the n >= 1 substeps
     for (int k = 1; k < n; ++k) {
-        R = R + (float)(k + 1) * A + 2.0f * q * q + zr * q;
-        float nzr = zr - s * q;
-        q = zr + q;
+        R = fmaf(zr, q, fmaf(__fmul_rn(2.0f, q), q, fmaf((float)(k + 1), A, R)));
+        const float nzr = fmaf(-s, q, zr);
+        q = __fadd_rn(zr, q);
         zr = nzr;
-        A = A * (1.0f + s);
+        A = __fmul_rn(A, s1);
     }
     // 1/A: the float estimate and one float64 Newton step
     double invA = (double)__fdividef(1.0f, A);
-    invA = invA * fma(-(double)A, invA, 2.0);
-    double C2 = (2.0 * zr) * q * invA;
-    double C3 = (2.0 * q) * q * invA;
-    double C1 = -(double)s * C3;
+    invA = __dmul_rn(invA, fma(-(double)A, invA, 2.0));
+    double C2 = __dmul_rn(__dmul_rn(2.0 * zr, q), invA);
+    double C3 = __dmul_rn(__dmul_rn(2.0 * q, q), invA);
+    double C1 = __dmul_rn(-(double)s, C3);
     // consistency in float64: scale (1 + C1, C2) onto the unit circle, then
     // C3 from C1 + C3 |t|^2 = 0
-    const double hg = 0.5 * fma(C1, 2.0 + C1, C2 * C2 * sd);
-    C1 = C1 - hg * (1.0 + C1);
-    C2 = C2 - hg * C2;
+    const double hg = __dmul_rn(0.5, fma(C1, __dadd_rn(2.0, C1), __dmul_rn(__dmul_rn(C2, C2), sd)));
+    C1 = fma(-hg, __dadd_rn(1.0, C1), C1);
+    C2 = fma(-hg, C2, C2);
     const float rs = s > 0.0f ? __fdividef(1.0f, s) : 0.0f;
-    C3 = C3 - fma(C3, sd, C1) * (double)rs;
-    return {t, e, C1, C2, C3, hasE ? (2.0 * R) * invA : 0.0};
+    C3 = fma(-fma(C3, sd, C1), (double)rs, C3);
+    return {t, e, C1, C2, C3, hasE ? __dmul_rn(2.0 * R, invA) : 0.0};
 }
 
 __device__ __forceinline__ D3 rotate_mixed(D3 v, const RotMixed& m, bool hasE) {
-    const D3 vxt = cross(v, m.t);
-    D3 dv = m.C1 * v + m.C2 * vxt + (m.C3 * dot(v, m.t)) * m.t;
-    if (hasE) dv = dv + m.C2 * m.e + m.C3 * cross(m.e, m.t) + (m.c6 * dot(m.e, m.t)) * m.t;
-    return v + dv;
+    D3 dv = axpy(__dmul_rn(m.C3, dot_fma(v, m.t)), m.t, axpy(m.C2, cross_fma(v, m.t), scale_rn(m.C1, v)));
+    if (hasE)
+        dv = axpy(__dmul_rn(m.c6, dot_fma(m.e, m.t)), m.t, axpy(m.C3, cross_fma(m.e, m.t), axpy(m.C2, m.e, dv)));
+    return {__dadd_rn(v.x, dv.x), __dadd_rn(v.y, dv.y), __dadd_rn(v.z, dv.z)};
 }
 
 __device__ __forceinline__ D3 rot_mixed(D3 v, D3 E, D3 B, double fac, int N, int n, bool hasE) {

@@ -203,6 +203,21 @@ __host__ __forceinline__ bool seg_config(const BorisArgs& a) {
     return (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP) && (fk == FK_DIPOLE || fk == FK_UNIFORM) && a.ppt != 2;
 }
 
+// fixed steps with E and B on one trilinear grid: the pair-gathering segment kernels,
+// except below 65536 particles with less than `dense` steps between saves.  There the
+// GPU is not full, and what counts is the latency of one step: a save takes a pass of
+// its own in the segment kernels, and the warps in it push the loop of the others out
+// of the instruction cache.  Measured, segment kernel and k_fixed* (device time, 20000
+// protons on 96^3 nodes between absorbing walls): FP32C Boris, 50 steps, saves every 2:
+// 168 and 136 us; 200 steps, every 10: 223 and 178; 400 steps, every 20: 171 and 177.
+// Float64: Boris, every 2: 195 and 170; every 5: 237 and 233; MultistepBoris4(2), every 5:
+// 625 and 489; every 10: 407 and 420.  200000 protons, every 2: FP32C 475 and 801,
+// float64 568 and 830.
+__host__ __forceinline__ bool ebgrid_seg_config(const BorisArgs& a, int dense) {
+    return (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP) && field_config_of(a.f) == FK_EBGRID &&
+           !(a.n < 65536 && a.save_everystep && a.ssi < dense);
+}
+
 // fixed steps, E zero and B on a trilinear uniform-Cartesian grid
 __host__ __forceinline__ bool gridb_config(const BorisArgs& a) {
     const DevField& B = a.f.B;
