@@ -1174,15 +1174,34 @@ int issue_boris_launch(tp_ctx* ctx, const tp_run_desc* d, BorisArgs& a, const La
     return TP_OK;
 }
 
-// Processing order of a solve in general Cartesian grids (n >= 65536): the
-// particles sorted by the Morton key of their initial cell, so that the lanes
-// of a warp gather neighbouring nodes (one radix sort of n keys, in the solve's
-// device time).  Results do not depend on the order.  Only the kernels that
-// gather lane by lane through the general evaluator gain (order 3, float64:
-// 1.07e9 -> 1.36e9 particle-steps/s).  The trilinear kernels and the
-// warp-cooperative cubic one do not: in order, 1e6 FP32C particles x 250 steps
-// took 5.37 ms against 5.73 sorted, and 100000 x 200 with every step saved 1.20
-// against 5.86, since the saves of a sorted warp scatter over the output rows.
+// Processing order of a solve in gridded fields (Cartesian geometry, n >= 65536): the
+// particles sorted by the Morton key of their initial cell, so that the lanes of a warp
+// gather neighbouring nodes (one radix sort of n keys, in the solve's device time).
+// Results do not depend on the order.  It pays where every lane gathers its own stencil
+// from more than one float table and saves are rare: a sorted warp's saves scatter over
+// the output rows, which costs as much as the sort gains at about one save in ten steps.
+// Device time in order and sorted, 1e6 protons x 250 steps, 2 saves, 128^3 nodes unless
+// stated:
+//   general grids (order 3, float64)              1.07e9 and 1.36e9 particle-steps/s
+//   E and B on grids, float64 nodes: float64      29.1 and 24.7 ms (Multistep 33.6, 29.3),
+//     float32 nodes of another type or geometry   27.8 and 23.1 (FP32C 20.9, 18.7),
+//     FP32C                                       13.1 and 12.7 (Multistep 14.0, 13.4),
+//     AdaptiveBoris, 500000 x 100                 7.58 and 7.10
+//   one grid and a uniform E, float64             16.1 and 14.5 (Multistep 20.0, 18.5)
+//   E and B, 100000 x 100, every step saved       1.51 and 2.24
+//   one grid, FP32C                               10.3 and 10.5
+//   one grid, AdaptiveBoris, 500000 x 100         4.34 and 4.28, FP32C 3.47 and 3.59
+//   E and B, float32 nodes, AdaptiveBoris         3.19 and 3.19
+// The pair-gathering and the cooperative cubic kernels gain nothing (FP32C 5.37 and 5.73).
+bool cell_order_pays(const tp_run_desc* d, const BorisArgs& a) {
+    const int fk = field_config_of(a.f);
+    if (fk == FK_GENGRID) return !(d->precision == TP_PREC_FP32C && fp32c_cubic_coop(a));
+    if (fk != FK_GENERIC || (d->save_everystep && d->savestepinterval < 16)) return false;
+    if (a.f.E.kind == TP_FIELD_GRID && a.f.B.kind == TP_FIELD_GRID) return true;
+    const bool adaptive = d->alg == TP_ALG_ADAPTIVE || d->alg == TP_ALG_ADAPTIVE_MULTISTEP;
+    return d->precision == TP_PREC_FP64 && !adaptive && !gridb_config(a);
+}
+
 // The scratch comes from the pool on stream s; the caller releases *buf
 // there after the push.
 int order_particles(tp_ctx* ctx, const tp_run_desc* d, BorisArgs& a, cudaStream_t s, void** buf) {
@@ -1192,7 +1211,7 @@ int order_particles(tp_ctx* ctx, const tp_run_desc* d, BorisArgs& a, cudaStream_
     if (a.f.B.kind == TP_FIELD_GRID && a.f.B.geom == TP_GRID_CARTESIAN) g = &a.f.B;
     else if (a.f.E.kind == TP_FIELD_GRID && a.f.E.geom == TP_GRID_CARTESIAN) g = &a.f.E;
     if (!g || a.n < 65536 || a.n > 0x7fffffffLL) return TP_OK;
-    if (field_config_of(a.f) != FK_GENGRID || (d->precision == TP_PREC_FP32C && fp32c_cubic_coop(a))) return TP_OK;
+    if (!cell_order_pays(d, a)) return TP_OK;
     size_t bytes = 0;
     cudaError_t e = cell_order(a.u0, a.n, *g, nullptr, &bytes, nullptr, s);
     if (e == cudaSuccess) e = cudaMallocAsync(buf, bytes, s);
