@@ -1008,7 +1008,7 @@ int tp_field_update(tp_field* f, const void* data) {
         std::lock_guard<std::mutex> lk(g_id_mu);
         f->id = g_next_id++;
     }
-    f->eb_partner = 0;
+    f->eb_partner = f->ebc_partner = 0;
     return TP_OK;
 }
 
