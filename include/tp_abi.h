@@ -479,7 +479,9 @@ int tp_autotune(tp_ctx* ctx, const tp_run_desc* desc, const tp_field* E,
 /* A full-orbit solve with fixed device buffers (the arguments of
  * tp_boris_run_device) captured once into a CUDA graph; tp_graph_launch
  * replays it on a stream.  Buffer contents may change between launches
- * (new initial states); the buffers and fields must outlive the graph.      */
+ * (new initial states), and a launch uses the fields' values of that time
+ * (tp_field_update); the buffers and fields must outlive the graph.  A launch
+ * after an update of E and B on one grid waits for the device once.         */
 typedef struct tp_graph tp_graph;
 int tp_boris_graph_create(tp_ctx* ctx, const tp_run_desc* desc,
                           const tp_field* E, const tp_field* B,

@@ -15,6 +15,7 @@
 #include <cstring>
 #include <limits>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <set>
 #include <string>
@@ -53,9 +54,12 @@ struct tp_ctx {
     int64_t done_cap = 0;
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t run_ev[2] = {nullptr, nullptr};
+    std::mutex pair_mu;  // the E/B tables that fields cache (tp_field::pair)
     // buffers of fields and tapes too large for the pool (held_alloc)
     std::set<void*> big;
 };
+
+struct PairTable;
 
 struct tp_field {
     tp_ctx* ctx = nullptr;
@@ -66,12 +70,7 @@ struct tp_field {
     void* d_raw = nullptr;   // uploaded (3, nx, ny, nz) data
     void* d_tab = nullptr;   // per-node table in the data's precision
     void* d_tab32 = nullptr; // float per-node table (only for f64 data)
-    // interleaved E/B table built on first use with a partner field
-    uint64_t eb_partner = 0;
-    void* d_eb32 = nullptr;
-    // the same for two cubic periodic grids (k_cubic32c)
-    uint64_t ebc_partner = 0;
-    void* d_ebc32 = nullptr;
+    std::shared_ptr<PairTable> pair;  // of the last E this field (as B) ran with
     void* d_axis[3] = {nullptr, nullptr, nullptr};  // node coordinates of non-uniform axes
     // SERIES: owned snapshot fields, their device descriptors and times
     std::vector<tp_field*> snaps;
@@ -613,6 +612,51 @@ DevTerm dev_term(const tp_term_desc& t) {
     return d;
 }
 
+}  // namespace
+
+// The float table with the nodes of E and B side by side (fields on one geometry).  The
+// field B caches the one of its last partner; runs, tapes and graphs hold theirs, so a
+// solve with another E leaves them what they read.
+struct PairTable {
+    tp_ctx* ctx;
+    const tp_field *E, *B;
+    uint64_t E_id, B_id;  // of the values in the table
+    bool cubic;
+    void* p = nullptr;
+    PairTable(tp_ctx* c, const tp_field* e, const tp_field* b, bool cub)
+        : ctx(c), E(e), B(b), E_id(e->id), B_id(b->id), cubic(cub) {}
+    PairTable(const PairTable&) = delete;
+    ~PairTable() {
+        if (!p) return;
+        DeviceGuard g(ctx->device);
+        cudaDeviceSynchronize();  // a launch on any stream may still read it
+        held_free(ctx, p);
+    }
+    bool current(const tp_field* e, const tp_field* b) const { return E_id == e->id && B_id == b->id; }
+    // the fields' present values; complete on return, since the entries that take the
+    // caller's stream are not ordered after the context's
+    cudaError_t pack() {
+        cudaStream_t s = ctx->stream;
+        const int f64e = E->desc.dtype == TP_DTYPE_F64, f64b = B->desc.dtype == TP_DTYPE_F64;
+        cudaError_t e;
+        if (cubic) {
+            e = launch_pack_node_table(E->d_raw, f64e, E->nodes, p, 0, 2, 0, s);
+            if (e == cudaSuccess) e = launch_pack_node_table(B->d_raw, f64b, B->nodes, p, 0, 2, 1, s);
+        } else {
+            e = launch_pack_eb(E->d_raw, B->d_raw, f64b, B->dev.n, p, s);
+        }
+        const cudaError_t done = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = done;
+        if (e == cudaSuccess) {
+            E_id = E->id;
+            B_id = B->id;
+        }
+        return e;
+    }
+};
+
+namespace {
+
 // the node tables of a grid from its raw data: x fastest for the general
 // evaluators, z fastest (tri_node) for the trilinear ones
 cudaError_t pack_tables(tp_field* f, bool f64, bool general, cudaStream_t s) {
@@ -626,46 +670,29 @@ cudaError_t pack_tables(tp_field* f, bool f64, bool general, cudaStream_t s) {
     return e;
 }
 
-// Build DevFields for a run; interleaves two grids on one geometry.
-int make_dev_fields(tp_ctx* ctx, const tp_field* E, tp_field* B, DevFields& F) {
+// Build DevFields for a run; interleaves two grids on one geometry.  `hold` keeps that
+// table alive: until the run's last launch, or as long as a tape or a graph may read it.
+int make_dev_fields(tp_ctx* ctx, const tp_field* E, tp_field* B, DevFields& F, std::shared_ptr<PairTable>& hold) {
     std::memset(&F, 0, sizeof(F));
     F.E = E->dev;
     F.B = B->dev;
-    if (same_geometry(E, B)) {
-        if (B->eb_partner != E->id) {
-            if (B->d_eb32) {
-                cudaDeviceSynchronize();  // a run on any stream may still read it
-                held_free(ctx, B->d_eb32);
-            }
-            B->d_eb32 = nullptr;
-            cudaError_t e = held_alloc(ctx, &B->d_eb32, (size_t)B->nodes * 8 * sizeof(float));
-            if (e == cudaSuccess)
-                e = launch_pack_eb(E->d_raw, B->d_raw, B->desc.dtype == TP_DTYPE_F64, B->dev.n, B->d_eb32, ctx->stream);
-            // the table is complete before any launch reads it: the entries
-            // that take the caller's stream are not ordered after this one
-            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "interleaved field table");
-            B->eb_partner = E->id;
-        }
-        F.eb_f64 = B->desc.dtype == TP_DTYPE_F64;
-        F.eb32 = (const float4*)B->d_eb32;
-    } else if (same_geometry_cubic(E, B)) {
-        if (B->ebc_partner != E->id) {
-            if (B->d_ebc32) {
-                cudaDeviceSynchronize();
-                held_free(ctx, B->d_ebc32);
-            }
-            B->d_ebc32 = nullptr;
-            const int f64e = E->desc.dtype == TP_DTYPE_F64, f64b = B->desc.dtype == TP_DTYPE_F64;
-            cudaError_t e = held_alloc(ctx, &B->d_ebc32, (size_t)B->nodes * 8 * sizeof(float));
-            if (e == cudaSuccess) e = launch_pack_node_table(E->d_raw, f64e, E->nodes, B->d_ebc32, 0, 2, 0, ctx->stream);
-            if (e == cudaSuccess) e = launch_pack_node_table(B->d_raw, f64b, B->nodes, B->d_ebc32, 0, 2, 1, ctx->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "interleaved cubic field table");
-            B->ebc_partner = E->id;
-        }
-        F.ebc32 = (const float4*)B->d_ebc32;
+    const bool cubic = same_geometry_cubic(E, B);
+    if (!cubic && !same_geometry(E, B)) {
+        hold.reset();
+        return TP_OK;
     }
+    std::lock_guard<std::mutex> lk(ctx->pair_mu);
+    if (!B->pair || !B->pair->current(E, B)) {
+        B->pair.reset();
+        auto t = std::make_shared<PairTable>(ctx, E, B, cubic);
+        cudaError_t e = held_alloc(ctx, &t->p, (size_t)B->nodes * 8 * sizeof(float));
+        if (e == cudaSuccess) e = t->pack();
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "interleaved field table");
+        B->pair = t;
+    }
+    hold = B->pair;
+    (cubic ? F.ebc32 : F.eb32) = (const float4*)hold->p;
+    if (!cubic) F.eb_f64 = B->desc.dtype == TP_DTYPE_F64;
     return TP_OK;
 }
 
@@ -1008,7 +1035,6 @@ int tp_field_update(tp_field* f, const void* data) {
         std::lock_guard<std::mutex> lk(g_id_mu);
         f->id = g_next_id++;
     }
-    f->eb_partner = f->ebc_partner = 0;
     return TP_OK;
 }
 
@@ -1016,7 +1042,7 @@ void tp_field_destroy(tp_field* f) {
     if (!f) return;
     DeviceGuard g(f->ctx->device);
     cudaDeviceSynchronize();  // a run on any stream may still read the field
-    for (void* p : {f->d_raw, f->d_tab, f->d_tab32, f->d_eb32, f->d_ebc32, f->d_axis[0], f->d_axis[1], f->d_axis[2],
+    for (void* p : {f->d_raw, f->d_tab, f->d_tab32, f->d_axis[0], f->d_axis[1], f->d_axis[2],
                     f->d_snaps, f->d_times, f->d_self})
         held_free(f->ctx, p);
     for (tp_field* c : f->snaps) tp_field_destroy(c);
@@ -1050,9 +1076,9 @@ namespace {
 
 // Fill the launch block of a full-orbit run (device pointers set by caller).
 int prepare_boris_args(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, tp_field* B,
-                       BorisArgs& a) {
+                       BorisArgs& a, std::shared_ptr<PairTable>& pair) {
     std::memset(&a, 0, sizeof(a));
-    int st = make_dev_fields(ctx, E, B, a.f);
+    int st = make_dev_fields(ctx, E, B, a.f, pair);
     if (st != TP_OK) return st;
     a.term = dev_term(d->term);
     a.alg = d->alg;
@@ -1313,7 +1339,8 @@ int tp_boris_run_device(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, co
         return fail(ctx, TP_E_ARG, "time step dt is too small, violating min_dt = 10 * eps(typeof(dt))");
     DeviceGuard g(ctx->device);
     BorisArgs a;
-    st = prepare_boris_args(ctx, d, E, const_cast<tp_field*>(B), a);
+    std::shared_ptr<PairTable> pair;
+    st = prepare_boris_args(ctx, d, E, const_cast<tp_field*>(B), a, pair);
     if (st != TP_OK) return st;
     cudaStream_t s = (cudaStream_t)stream;
     // the interleaved table (if any) was built on the context stream
@@ -1382,7 +1409,8 @@ int tp_autotune(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, const tp_f
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return fail(ctx, TP_E_NOMEM, std::string("autotune buffers: ") + cudaGetErrorString(e));
     BorisArgs a;
-    st = prepare_boris_args(ctx, &ds, E, const_cast<tp_field*>(B), a);
+    std::shared_ptr<PairTable> pair;
+    st = prepare_boris_args(ctx, &ds, E, const_cast<tp_field*>(B), a, pair);
     if (st != TP_OK) return st;
     e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "field table");
@@ -1484,6 +1512,7 @@ struct tp_graph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     unsigned long long* queue = nullptr;
+    std::shared_ptr<PairTable> pair;
     ~tp_graph() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -1510,7 +1539,8 @@ int tp_boris_graph_create(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, 
         return fail(ctx, TP_E_ARG, "time step dt is too small, violating min_dt = 10 * eps(typeof(dt))");
     DeviceGuard g(ctx->device);
     BorisArgs a;
-    st = prepare_boris_args(ctx, d, E, const_cast<tp_field*>(B), a);
+    std::shared_ptr<PairTable> pair;
+    st = prepare_boris_args(ctx, d, E, const_cast<tp_field*>(B), a, pair);
     if (st != TP_OK) return st;
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "field table");
@@ -1530,6 +1560,7 @@ int tp_boris_graph_create(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, 
     if (st != TP_OK) return st;
     auto* gr = new tp_graph();
     gr->ctx = ctx;
+    gr->pair = pair;
     if (a.use_queue) {
         e = cudaMalloc((void**)&gr->queue, sizeof(unsigned long long));
         if (e != cudaSuccess) {
@@ -1564,7 +1595,16 @@ int tp_boris_graph_create(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, 
 int tp_graph_launch(tp_graph* gr, void* stream) {
     if (!gr) return TP_E_ARG;
     DeviceGuard g(gr->ctx->device);
-    cudaError_t e = cudaGraphLaunch(gr->exec, (cudaStream_t)stream);
+    cudaError_t e = cudaSuccess;
+    if (gr->pair) {  // a field was updated: the graph's table takes the new values, as its other tables have
+        std::lock_guard<std::mutex> lk(gr->ctx->pair_mu);
+        if (!gr->pair->current(gr->pair->E, gr->pair->B)) {
+            e = cudaDeviceSynchronize();
+            if (e == cudaSuccess) e = gr->pair->pack();
+            if (e != cudaSuccess) return cuda_fail(gr->ctx, e, "interleaved field table");
+        }
+    }
+    e = cudaGraphLaunch(gr->exec, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(gr->ctx, e, "graph launch");
     return TP_OK;
 }
@@ -1635,7 +1675,8 @@ int tp_boris_run(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, const tp_
             return cuda_fail(ctx, e, "input upload");
         }
         BorisArgs a;
-        st = prepare_boris_args(ctx, d, E, const_cast<tp_field*>(B), a);
+        std::shared_ptr<PairTable> pair;
+        st = prepare_boris_args(ctx, d, E, const_cast<tp_field*>(B), a, pair);
         if (st != TP_OK) {
             delete r;
             return st;
@@ -1821,7 +1862,8 @@ int run_host_once(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, tp_field
     }
     std::memset(h + o_zero, 0, 64);
     BorisArgs a;
-    int st = prepare_boris_args(ctx, d, E, B, a);
+    std::shared_ptr<PairTable> pair;
+    int st = prepare_boris_args(ctx, d, E, B, a, pair);
     if (st != TP_OK) return st;
     a.n = n;
     a.nslots = nslots;
@@ -1970,7 +2012,8 @@ int tp_boris_run_host(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, cons
             return cuda_fail(ctx, e, "input upload");
         }
         BorisArgs a;
-        st = prepare_boris_args(ctx, d, E, const_cast<tp_field*>(B), a);
+        std::shared_ptr<PairTable> pair;
+        st = prepare_boris_args(ctx, d, E, const_cast<tp_field*>(B), a, pair);
         if (st != TP_OK) {
             cudaStreamSynchronize(s);
             return st;
@@ -2852,6 +2895,7 @@ struct tp_tape {
     const tp_field* E = nullptr;
     const tp_field* B = nullptr;
     uint64_t E_id = 0, B_id = 0;
+    std::shared_ptr<PairTable> pair;
     AdjArgs A{};
     int fk = 0;
     LaunchCfg cfg{};
@@ -2924,7 +2968,7 @@ int adjoint_prepare(tp_ctx* ctx, const tp_adj_desc* d, const tp_field* E, const 
     t->E_id = E->id;
     t->B_id = B->id;
     AdjArgs& A = t->A;
-    st = prepare_boris_args(ctx, r, E, const_cast<tp_field*>(B), A.a);
+    st = prepare_boris_args(ctx, r, E, const_cast<tp_field*>(B), A.a, t->pair);
     if (st != TP_OK) {
         delete t;
         return st;
@@ -3162,7 +3206,7 @@ int tp_tape_rerun_device(tp_tape* t, const double* u0, double* u_final, void* st
     DeviceGuard g(ctx->device);
     // refresh the field tables: a field may have been updated since the recording
     DevFields f;
-    int st = make_dev_fields(ctx, t->E, const_cast<tp_field*>(t->B), f);
+    int st = make_dev_fields(ctx, t->E, const_cast<tp_field*>(t->B), f, t->pair);
     if (st != TP_OK) return st;
     t->A.a.f = f;
     t->E_id = t->E->id;
