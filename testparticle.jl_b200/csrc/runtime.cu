@@ -54,6 +54,7 @@ struct tp_ctx {
     int64_t done_cap = 0;
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t run_ev[2] = {nullptr, nullptr};
+    cudaMemPool_t held = nullptr;  // fields and tapes (held_alloc)
     std::mutex pair_mu;  // the E/B tables that fields cache (tp_field::pair)
     // buffers of fields and tapes too large for the pool (held_alloc)
     std::set<void*> big;
@@ -162,15 +163,16 @@ struct DBuf {
 };
 
 // Device memory that outlives a call (field tables, adjoint tapes).  Buffers of up
-// to 2 GB come from the pool, which keeps what is released for the next field or
-// tape (creating and freeing them with cudaMalloc / cudaFree took two thirds of a
-// differentiated solve of 131072 particles x 128 steps); larger ones go back to
-// the driver at once.  A buffer may be used on any stream once held_ready has
-// returned; before held_free the caller makes sure that no stream uses it.
+// to 2 GB come from a pool of the context, which keeps at most 2 GB of what is released
+// for the next field or tape (creating and freeing them with cudaMalloc / cudaFree took
+// two thirds of a differentiated solve of 131072 particles x 128 steps); larger ones go
+// back to the driver at once.  A buffer may be used on any stream once held_ready has
+// returned; before held_free the caller makes sure that no stream uses it, and after the
+// last one it calls held_trim.
 constexpr size_t kPoolMax = (size_t)2 << 30;
 
 cudaError_t held_alloc(tp_ctx* ctx, void** p, size_t bytes) {
-    if (bytes <= kPoolMax) return cudaMallocAsync(p, bytes, ctx->stream);
+    if (bytes <= kPoolMax) return cudaMallocFromPoolAsync(p, bytes, ctx->held, ctx->stream);
     const cudaError_t e = cudaMalloc(p, bytes);
     if (e == cudaSuccess) ctx->big.insert(*p);
     return e;
@@ -184,17 +186,34 @@ void held_free(tp_ctx* ctx, void* p) {
     else cudaFreeAsync(p, ctx->stream);
 }
 
+// bytes the pool holds beyond those in use, which it reports in `used`
+uint64_t unused_memory(cudaMemPool_t pool, uint64_t* used) {
+    uint64_t held = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return held > *used ? held - *used : 0;
+}
+
+void held_trim(tp_ctx* ctx) {
+    uint64_t used = 0;
+    if (unused_memory(ctx->held, &used) <= kPoolMax) return;
+    cudaStreamSynchronize(ctx->stream);
+    cudaMemPoolTrimTo(ctx->held, used + kPoolMax);
+    cudaGetLastError();
+}
+
 // device memory a large allocation can have: what the driver has free and what
-// the pool holds unused
+// the pools hold unused
 size_t free_memory(tp_ctx* ctx) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     cudaMemPool_t pool;
-    uint64_t held = 0, used = 0;
-    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
-        free_b += held - used;
+    uint64_t used = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess) free_b += unused_memory(pool, &used);
+    free_b += unused_memory(ctx->held, &used);
     cudaGetLastError();
     return free_b;
 }
@@ -684,6 +703,7 @@ int make_dev_fields(tp_ctx* ctx, const tp_field* E, tp_field* B, DevFields& F, s
     std::lock_guard<std::mutex> lk(ctx->pair_mu);
     if (!B->pair || !B->pair->current(E, B)) {
         B->pair.reset();
+        held_trim(ctx);
         auto t = std::make_shared<PairTable>(ctx, E, B, cubic);
         cudaError_t e = held_alloc(ctx, &t->p, (size_t)B->nodes * 8 * sizeof(float));
         if (e == cudaSuccess) e = t->pack();
@@ -803,6 +823,15 @@ int tp_ctx_create(int device, tp_ctx** out) {
     e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        e = cudaMemPoolCreate(&c->held, &props);
+        uint64_t keep = UINT64_MAX;  // held_trim bounds it
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(c->held, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    if (e == cudaSuccess) {
         // keep freed pool memory in this process for the next solve
         cudaMemPool_t pool;
         if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
@@ -812,6 +841,8 @@ int tp_ctx_create(int device, tp_ctx** out) {
         cudaGetLastError();
     }
     if (e != cudaSuccess) {
+        if (c->held) cudaMemPoolDestroy(c->held);
+        if (c->stream) cudaStreamDestroy(c->stream);
         delete c;
         cudaGetLastError();
         return TP_E_CUDA;
@@ -837,6 +868,7 @@ void tp_ctx_destroy(tp_ctx* ctx) {
     for (cudaEvent_t ev : ctx->run_ev)
         if (ev) cudaEventDestroy(ev);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    cudaMemPoolDestroy(ctx->held);
     delete ctx;
 }
 
@@ -1046,7 +1078,9 @@ void tp_field_destroy(tp_field* f) {
                     f->d_snaps, f->d_times, f->d_self})
         held_free(f->ctx, p);
     for (tp_field* c : f->snaps) tp_field_destroy(c);
+    tp_ctx* ctx = f->ctx;
     delete f;
+    held_trim(ctx);
 }
 
 int tp_boris_slots(const tp_run_desc* d, const double* dt_i, const double* tend_i, int64_t n,
@@ -1611,9 +1645,11 @@ int tp_graph_launch(tp_graph* gr, void* stream) {
 
 void tp_graph_destroy(tp_graph* gr) {
     if (!gr) return;
-    DeviceGuard g(gr->ctx->device);
+    tp_ctx* ctx = gr->ctx;
+    DeviceGuard g(ctx->device);
     cudaDeviceSynchronize();
     delete gr;
+    held_trim(ctx);
 }
 
 int tp_boris_run(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, const tp_field* B,
@@ -3231,9 +3267,11 @@ int tp_tape_segments(const tp_tape* t, int64_t* checkpoint_every, int64_t* segme
 void tp_tape_destroy(tp_tape* t) {
     if (!t) return;
     DeviceGuard g(t->ctx->device);
-    cudaStreamSynchronize(t->ctx->stream);
+    tp_ctx* ctx = t->ctx;
+    cudaStreamSynchronize(ctx->stream);
     cudaDeviceSynchronize();
     delete t;
+    held_trim(ctx);
 }
 
 }  // extern "C"
