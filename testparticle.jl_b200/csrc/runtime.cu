@@ -56,7 +56,9 @@ struct tp_ctx {
     cudaEvent_t run_ev[2] = {nullptr, nullptr};
     cudaMemPool_t held = nullptr;  // fields and tapes (held_alloc)
     std::mutex pair_mu;  // the E/B tables that fields cache (tp_field::pair)
-    // buffers of fields and tapes too large for the pool (held_alloc)
+    // buffers of fields and tapes too large for the pool (held_alloc); Python may
+    // destroy a tape or a field on any thread
+    std::mutex big_mu;
     std::set<void*> big;
 };
 
@@ -174,7 +176,9 @@ constexpr size_t kPoolMax = (size_t)2 << 30;
 cudaError_t held_alloc(tp_ctx* ctx, void** p, size_t bytes) {
     if (bytes <= kPoolMax) return cudaMallocFromPoolAsync(p, bytes, ctx->held, ctx->stream);
     const cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaSuccess) ctx->big.insert(*p);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(ctx->big_mu);
+    ctx->big.insert(*p);
     return e;
 }
 
@@ -182,7 +186,12 @@ cudaError_t held_ready(tp_ctx* ctx) { return cudaStreamSynchronize(ctx->stream);
 
 void held_free(tp_ctx* ctx, void* p) {
     if (!p) return;
-    if (ctx->big.erase(p)) cudaFree(p);
+    bool big;
+    {
+        std::lock_guard<std::mutex> lk(ctx->big_mu);
+        big = ctx->big.erase(p) > 0;
+    }
+    if (big) cudaFree(p);
     else cudaFreeAsync(p, ctx->stream);
 }
 
