@@ -42,7 +42,9 @@ struct tp_ctx {
         int block, sched, ppt;
     };
     std::map<std::string, Shape> tuned;
-    // pinned staging for host <-> device transfers of pageable buffers
+    // pinned staging for host <-> device transfers of pageable buffers.  A copy that may
+    // still be in flight when a transfer returns has recorded the buffer's event, and
+    // every transfer waits for it before it writes to the buffer (staging_idle)
     void* pin[2] = {nullptr, nullptr};
     cudaEvent_t pin_ev[2] = {nullptr, nullptr};
     // tp_boris_run_host, created on first use and kept: pinned staging of
@@ -290,6 +292,15 @@ cudaError_t ensure_chunk_pin(tp_ctx* ctx, size_t bytes) {
     return e;
 }
 
+cudaError_t staging_idle(tp_ctx* ctx) {
+    for (cudaEvent_t ev : ctx->pin_ev)
+        if (ev) {
+            const cudaError_t e = cudaEventSynchronize(ev);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
 bool is_pageable(const void* p) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -316,6 +327,7 @@ cudaError_t copy_to_host_on(tp_ctx* ctx, cudaStream_t s, void* dst, const void* 
         return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
     }
     cudaError_t e = ensure_pinned(ctx);
+    if (e == cudaSuccess) e = staging_idle(ctx);
     if (e != cudaSuccess) return e;
     const size_t nch = (bytes + kPinChunk - 1) / kPinChunk;
     for (size_t k = 0; k <= nch; ++k) {
@@ -346,6 +358,7 @@ cudaError_t copy_to_device_on(tp_ctx* ctx, cudaStream_t s, void* dst, const void
     if (bytes == 0) return cudaSuccess;
     if (bytes < ((size_t)4 << 20) || !is_pageable(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, s);
     cudaError_t e = ensure_pinned(ctx);
+    if (e == cudaSuccess) e = staging_idle(ctx);
     if (e != cudaSuccess) return e;
     const size_t nch = (bytes + kPinChunk - 1) / kPinChunk;
     for (size_t k = 0; k < nch; ++k) {
@@ -385,7 +398,7 @@ char* staging(tp_ctx* ctx, size_t bytes) {
     if (bytes == 0 || bytes > kPinChunk) return nullptr;
     cudaError_t e = cudaSuccess;
     void* p = ctx->pin[0];
-    if (!p && bytes <= ((size_t)8 << 20)) {
+    if (!p && bytes < ((size_t)8 << 20)) {
         size_t room = (size_t)256 << 10;
         while (room < bytes) room *= 2;
         e = ensure_chunk_pin(ctx, room);
@@ -394,13 +407,13 @@ char* staging(tp_ctx* ctx, size_t bytes) {
         e = ensure_pinned(ctx, 1);
         p = ctx->pin[0];
     }
+    if (e == cudaSuccess) e = staging_idle(ctx);
     if (e == cudaSuccess) return (char*)p;
     cudaGetLastError();
     return nullptr;
 }
 
-// host -> device on stream s, asynchronous (the caller synchronises s before it
-// returns).  Below 8 MB in all the arrays go one by one, which takes the driver's own
+// host -> device on stream s, asynchronous.  Below 8 MB in all the arrays go one by one, which takes the driver's own
 // staging: no destination page is touched for the first time here, and starting
 // the threads costs more (60000 guiding centres, 3.8 MB: 0.4 ms)
 cudaError_t upload_parts(tp_ctx* ctx, cudaStream_t s, const std::vector<Part>& parts) {
@@ -425,6 +438,10 @@ cudaError_t upload_parts(tp_ctx* ctx, cudaStream_t s, const std::vector<Part>& p
     host_copies(copies);
     for (const Part& p : dma)
         if (e == cudaSuccess) e = cudaMemcpyAsync(p.dst, p.src, p.bytes, cudaMemcpyHostToDevice, s);
+    if (!dma.empty()) {
+        const cudaError_t r = cudaEventRecord(ctx->pin_ev[0], s);
+        if (e == cudaSuccess) e = r;
+    }
     return e;
 }
 
