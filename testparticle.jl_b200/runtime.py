@@ -322,7 +322,8 @@ class Context:
             nsteps = np.empty(n.value, dtype=np.int64)
             t = np.empty(tot.value, dtype=np.float64)
             u = np.empty((tot.value, w.value), dtype=np.float64)
-            lib.tp_result_copy(res, _ptr(nsaved), _ptr(retcode), _ptr(nsteps), _ptr(t), _ptr(u))
+            _check(lib, self.handle, lib.tp_result_copy(res, _ptr(nsaved), _ptr(retcode), _ptr(nsteps), _ptr(t), _ptr(u)),
+                   "tp_result_copy")
             ms = C.c_double()
             lib.tp_result_elapsed_ms(res, C.byref(ms))
         finally:
