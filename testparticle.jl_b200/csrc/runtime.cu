@@ -3199,7 +3199,7 @@ int tp_adjoint_forward_device(tp_ctx* ctx, const tp_adj_desc* d, const tp_field*
     DeviceGuard g(ctx->device);
     st = adjoint_forward_on(t, u0, u_final, (cudaStream_t)stream);
     if (st != TP_OK) {
-        delete t;
+        tp_tape_destroy(t);  // waits: the copy of u0 may still be on its way into the tape
         return st;
     }
     *tape = t;
@@ -3237,7 +3237,7 @@ int tp_adjoint_forward(tp_ctx* ctx, const tp_adj_desc* d, const tp_field* E, con
         if (e != cudaSuccess) st = cuda_fail(ctx, e, "adjoint forward");
     }
     if (st != TP_OK) {
-        delete t;
+        tp_tape_destroy(t);
         return st;
     }
     *tape = t;
