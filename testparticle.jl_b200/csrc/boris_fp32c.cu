@@ -765,19 +765,12 @@ static const void* pick_fk32(bool adaptive, int fk, int ppt) {
     return kernel_ptr32<MULTI, QUEUE, FK_GENERIC>(adaptive, 1);
 }
 
-// fixed steps in static cubic grids with the interleaved table
-static bool cubic_coop_kernel(const BorisArgs& a) {
-    return a.f.ebc32 != nullptr && (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP);
-}
-
-bool fp32c_cubic_coop(const BorisArgs& a) { return cubic_coop_kernel(a); }
-
 static const void* select_kernel32(const BorisArgs& a, bool queue) {
     const bool multi = a.alg == TP_ALG_MULTISTEP || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
-    if (cubic_coop_kernel(a)) return multi ? (const void*)k_cubic32c<true> : (const void*)k_cubic32c<false>;
+    if (cubic_coop_config(a)) return multi ? (const void*)k_cubic32c<true> : (const void*)k_cubic32c<false>;
     if (seg_config(a)) return seg_kernel32(a, queue);
-    if (ebgrid_seg_config(a, 16)) return grid_kernel32(a, queue);
+    if (ebgrid_seg_config(a, true)) return grid_kernel32(a, queue);
     const int fk = field_config_of(a.f);
     const int ppt = a.ppt;
     if (multi) return queue ? pick_fk32<true, true>(adaptive, fk, ppt) : pick_fk32<true, false>(adaptive, fk, ppt);

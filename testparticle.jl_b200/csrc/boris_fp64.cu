@@ -441,7 +441,7 @@ static const void* pick_fk64(bool adaptive, const BorisArgs& a) {
 
 static const void* select_kernel64(const BorisArgs& a, bool queue) {
     if (seg_config(a)) return seg_kernel64(a, queue);
-    if (ebgrid_seg_config(a, a.alg == TP_ALG_MULTISTEP ? 8 : 4)) return grid_kernel64(a, queue);
+    if (ebgrid_seg_config(a, false)) return grid_kernel64(a, queue);
     if (gridb_config(a)) return gridb_kernel64(a, queue);
     const bool multi = a.alg == TP_ALG_MULTISTEP || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;
     const bool adaptive = a.alg == TP_ALG_ADAPTIVE || a.alg == TP_ALG_ADAPTIVE_MULTISTEP;

@@ -1196,7 +1196,7 @@ int prepare_boris_args(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, tp_
 // key of the kernel variant a run selects (what tp_autotune tunes)
 std::string tune_key(const tp_run_desc* d, const BorisArgs& a) {
     return std::to_string(d->alg) + ":" + std::to_string(d->precision) + ":" +
-           std::to_string(field_config_of(a.f)) + ":" + std::to_string(d->term.flags != 0);
+           std::to_string(kernel_variant(a, d->precision == TP_PREC_FP32C)) + ":" + std::to_string(d->term.flags != 0);
 }
 
 // Effective block size, schedule and particles per thread of a run: the
@@ -1243,7 +1243,7 @@ int plan_boris_launch(tp_ctx* ctx, const tp_run_desc* d, BorisArgs& a, LaunchCfg
     resolve_launch(ctx, d, a, block, q, ppt);
     if (ppt != 1 && ppt != 2) return fail(ctx, TP_E_ARG, "particles_per_thread must be 0, 1 or 2");
     if (ppt == 2 && !ppt2_available(d, a)) ppt = 1;
-    if (d->precision == TP_PREC_FP32C && fp32c_cubic_coop(a)) {
+    if (d->precision == TP_PREC_FP32C && cubic_coop_config(a)) {
         q = false;  // the warp-cooperative kernel walks one particle per lane, static
         if (block > 128) block = 128;
     }
@@ -1310,7 +1310,7 @@ int issue_boris_launch(tp_ctx* ctx, const tp_run_desc* d, BorisArgs& a, const La
 // The pair-gathering and the cooperative cubic kernels gain nothing (FP32C 5.37 and 5.73).
 bool cell_order_pays(const tp_run_desc* d, const BorisArgs& a) {
     const int fk = field_config_of(a.f);
-    if (fk == FK_GENGRID) return !(d->precision == TP_PREC_FP32C && fp32c_cubic_coop(a));
+    if (fk == FK_GENGRID) return !(d->precision == TP_PREC_FP32C && cubic_coop_config(a));
     if (fk != FK_GENERIC || (d->save_everystep && d->savestepinterval < 16)) return false;
     if (a.f.E.kind == TP_FIELD_GRID && a.f.B.kind == TP_FIELD_GRID) return true;
     const bool adaptive = d->alg == TP_ALG_ADAPTIVE || d->alg == TP_ALG_ADAPTIVE_MULTISTEP;

@@ -213,7 +213,8 @@ __host__ __forceinline__ bool seg_config(const BorisArgs& a) {
 // Float64: Boris, every 2: 195 and 170; every 5: 237 and 233; MultistepBoris4(2), every 5:
 // 625 and 489; every 10: 407 and 420.  200000 protons, every 2: FP32C 475 and 801,
 // float64 568 and 830.
-__host__ __forceinline__ bool ebgrid_seg_config(const BorisArgs& a, int dense) {
+__host__ __forceinline__ bool ebgrid_seg_config(const BorisArgs& a, bool fp32c) {
+    const int dense = fp32c ? 16 : a.alg == TP_ALG_MULTISTEP ? 8 : 4;
     return (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP) && field_config_of(a.f) == FK_EBGRID &&
            !(a.n < 65536 && a.save_everystep && a.ssi < dense);
 }
@@ -223,6 +224,20 @@ __host__ __forceinline__ bool gridb_config(const BorisArgs& a) {
     const DevField& B = a.f.B;
     return (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP) && a.f.E.kind == TP_FIELD_ZERO &&
            B.kind == TP_FIELD_GRID && !B.general;
+}
+
+// E and B on one periodic cubic grid, FP32C: four lanes per particle (k_cubic32c)
+__host__ __forceinline__ bool cubic_coop_config(const BorisArgs& a) {
+    return a.f.ebc32 != nullptr && (a.alg == TP_ALG_BORIS || a.alg == TP_ALG_MULTISTEP);
+}
+
+// The kernels that a run of one algorithm and precision selects among, whatever its launch
+// shape: a shape tuned for one (tp_autotune) says nothing about another.
+__host__ __forceinline__ int kernel_variant(const BorisArgs& a, bool fp32c) {
+    if (fp32c && cubic_coop_config(a)) return 8;
+    if (!fp32c && gridb_config(a)) return 7;
+    if (ebgrid_seg_config(a, fp32c)) return 6;
+    return kernel_config_of(a.f);
 }
 
 // particle i's outputs are final: publish them, then count the particle

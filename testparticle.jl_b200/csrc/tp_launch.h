@@ -171,8 +171,6 @@ cudaError_t launch_eb_unpack(const float4* tab, const int32_t n[3], int off, int
 
 cudaError_t launch_boris_fp64(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s);
 cudaError_t launch_boris_fp32c(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s);
-// the FP32C run takes the warp-cooperative cubic-grid kernel (static schedule only)
-bool fp32c_cubic_coop(const BorisArgs& a);
 int occupancy_boris_fp64(const BorisArgs& a, int block);
 int occupancy_boris_fp32c(const BorisArgs& a, int block);
 
