@@ -366,8 +366,10 @@ function collect_result(ctx, res, prob, alg_name, T)
     ccall((:tp_result_info, libtpb200), Cint, (Ptr{Cvoid}, Ref{Int64}, Ref{Int32}, Ref{Int64}), res, n, w, tot)
     ns = Vector{Int32}(undef, n[]); rc = Vector{Int8}(undef, n[]); st = Vector{Int64}(undef, n[])
     t = Vector{Float64}(undef, tot[]); u = Matrix{Float64}(undef, w[], tot[])
-    ccall((:tp_result_copy, libtpb200), Cint, (Ptr{Cvoid}, Ptr{Int32}, Ptr{Int8}, Ptr{Int64}, Ptr{Float64}, Ptr{Float64}),
-        res, ns, rc, st, t, u)
+    code = ccall((:tp_result_copy, libtpb200), Cint,
+        (Ptr{Cvoid}, Ptr{Int32}, Ptr{Int8}, Ptr{Int64}, Ptr{Float64}, Ptr{Float64}), res, ns, rc, st, t, u)
+    code == 0 || ccall((:tp_result_destroy, libtpb200), Cvoid, (Ptr{Cvoid},), res)
+    check(ctx, code, "tp_result_copy")
     ms = Ref{Float64}(0.0)
     ccall((:tp_result_elapsed_ms, libtpb200), Cint, (Ptr{Cvoid}, Ref{Float64}), res, ms)
     ccall((:tp_result_destroy, libtpb200), Cvoid, (Ptr{Cvoid},), res)
