@@ -1903,7 +1903,8 @@ int64_t pack_chunk_host(const double* t_st, const double* u_st, const int32_t* n
     return off[m];
 }
 
-// tp_boris_run_host for an ensemble of one chunk: inputs, counters and results lie
+// tp_boris_run_host for an ensemble of one chunk (below 65536 particles, so in its own
+// order): inputs, counters and results lie
 // in one device buffer with a pinned mirror, so the solve is one allocation, one
 // copy in, the launch, one copy out and one wait.  (Eleven allocations, as many
 // small copies, and polling at 250 us made 0.33 ms of the 0.45 ms that one orbit
@@ -1960,11 +1961,8 @@ int run_host_once(tp_ctx* ctx, const tp_run_desc* d, const tp_field* E, tp_field
     for (int k = 0; k < 3; ++k)
         if (e == cudaSuccess && direct[k]) e = cudaMemcpyAsync(in[k].dst, in[k].src, in[k].bytes, cudaMemcpyDefault, s);
     if (e == cudaSuccess) e = cudaEventRecord(ctx->run_ev[0], s);
-    void* obuf = nullptr;
     if (e == cudaSuccess) {
-        st = order_particles(ctx, d, a, s, &obuf);
-        if (st == TP_OK) st = launch_boris(ctx, d, a, s, (unsigned long long*)(p + o_zero + 8));
-        if (obuf) cudaFreeAsync(obuf, s);
+        st = launch_boris(ctx, d, a, s, (unsigned long long*)(p + o_zero + 8));
         e = cudaEventRecord(ctx->run_ev[1], s);
     }
     if (e == cudaSuccess && st == TP_OK) e = cudaMemcpyAsync(h + o_zero, p + o_zero, end - o_zero, cudaMemcpyDeviceToHost, s);
