@@ -518,10 +518,11 @@ __global__ void __launch_bounds__(256) k_adj_forward(AdjArgs A) {
 // (pair_gather.cuh): a warp takes 32 particles and stays together.  The dot
 // products are contracted as in k_adj_forward, so the final states and the tape
 // equal its bits.  Bound by L1 line look-ups, 5 per particle and step instead of 8.
-// Forward and backward of 131072 protons x 128 steps on 128^3 nodes: 3.93 -> 3.30
-// ms with a register cap of 896 threads, which takes the 1024 blocks in one wave;
-// 512 3.40, 256 3.55, 640 3.48, 768 3.49.  512 is faster for fewer (20000: 1.44
-// against 1.52, 60000: 2.2 against 2.3) and equal for 300000 (6.05).
+// Forward and backward of 131072 protons x 128 steps on 128^3 nodes, before the reductions
+// of the backward were reordered: 3.93 -> 3.40 ms with this register cap of 512 threads;
+// 256 3.55, 640 3.48, 768 3.49, and 896, which takes the 1024 blocks in one wave, 3.30.
+// 512 is faster for fewer (20000: 1.44 against 1.52, 60000: 2.2 against 2.3) and equal for
+// 300000 (6.05).
 template <bool PERIODIC>
 __global__ void __launch_bounds__(512, 1) k_adj_forward_eb(const __grid_constant__ AdjArgs A) {
     const BorisArgs& a = A.a;
@@ -806,10 +807,13 @@ __device__ __forceinline__ void scatter_warp_eb(const AdjArgs& A, float* stage, 
         tri_nodes_eb(g, ax, ay, az, nd);
         tri_weights(ax, ay, az, w);
         float4* me = reinterpret_cast<float4*>(stage + lane * kStage);
-        me[0] = make_float4(__int_as_float(nd[0]), __int_as_float(nd[1]), __int_as_float(nd[2]), __int_as_float(nd[3]));
-        me[1] = make_float4(__int_as_float(nd[4]), __int_as_float(nd[5]), __int_as_float(nd[6]), __int_as_float(nd[7]));
-        me[2] = make_float4(w[0], w[1], w[2], w[3]);
-        me[3] = make_float4(w[4], w[5], w[6], w[7]);
+        // z neighbours first: they are next to each other in the table, and eight lanes of a
+        // reduction then touch two runs of 64 bytes instead of four nodes (131072 protons x
+        // 128 steps: backward 2.26 -> 2.15 ms; 2^18 x 4096 111.2 -> 107.0)
+        me[0] = make_float4(__int_as_float(nd[0]), __int_as_float(nd[4]), __int_as_float(nd[2]), __int_as_float(nd[6]));
+        me[1] = make_float4(__int_as_float(nd[1]), __int_as_float(nd[5]), __int_as_float(nd[3]), __int_as_float(nd[7]));
+        me[2] = make_float4(w[0], w[4], w[2], w[6]);
+        me[3] = make_float4(w[1], w[5], w[3], w[7]);
         me[4] = make_float4(ct.lE.x, ct.lE.y, ct.lE.z, 0.0f);
         me[5] = make_float4(ct.lB.x, ct.lB.y, ct.lB.z, 0.0f);
     }
