@@ -55,7 +55,7 @@ TRAFFIC_PER_PARTICLE_STEP = 8.4
 # one warp-step of the dipole's segment kernel issues and the DRAM bytes per
 # particle-step, both measured by ncu
 FLOPS_PER_PARTICLE_STEP_DIPOLE = 150
-INST_PER_WARP_STEP_DIPOLE = 249.0
+INST_PER_WARP_STEP_DIPOLE = 253.0
 TRAFFIC_PER_PARTICLE_STEP_DIPOLE = 0.32
 PEAKS_FILE = ROOT / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6650.0

@@ -5,13 +5,13 @@
 // vel_update64 bit for bit.
 //
 // Measured on the device, 400009 protons x 250 steps on a 120 x 100 x 91 grid:
-// Boris 4.72 -> 2.55 ms, MultistepBoris4(2) 6.42 -> 4.07 ms (2.79 while the
-// particles were still sorted by cell first).  A Boris step is 457
-// warp instructions, 206 on the float64 pipe and 58 on the XU (float to float64
-// conversions); L1 is 70 % busy with 5 line look-ups per particle.
+// Boris 4.72 -> 2.51 ms, MultistepBoris4(2) 6.42 -> 4.07 ms (Boris 2.79 while the
+// particles were still sorted by cell first).  A Boris step is 474 warp
+// instructions, 206 on the float64 pipe and 58 on the XU (float to float64
+// conversions); L1 is 71 % busy with 5 line look-ups per particle.
 //
 // B alone, float64 data, 61 x 53 x 47 nodes, 250 steps between absorbing walls:
-// 200003 protons, Boris 2.89 -> 1.09 ms, MultistepBoris4(2) 8.81 -> 1.65;
+// 200003 protons, Boris 2.89 -> 1.01 ms, MultistepBoris4(2) 8.81 -> 1.65;
 // 400000, Boris 6.33 -> 1.89; 20000 0.47 -> 0.38.  k_fixed64 read a stencil with
 // 16 loads of 32 lines each and decided on the field kinds in every step.
 #include "boris64_common.cuh"

@@ -7,8 +7,8 @@
 // Measured on the device against the general kernels, dipole, 1e6 protons x 1000
 // steps: MultistepBoris4(2) 12.44 -> 9.03 ms, Boris 10.93 -> 7.73 ms; 300001
 // protons with AdaptiveBoris(0.1) of at most 1000 steps 4.81 -> 4.04 ms.  A
-// Multistep step is 249 warp instructions (341 before): 87 on the float64 pipe,
-// 73 FMA, 38 ALU, 23 XU (float <-> float64 conversions); issue is 70 % busy,
+// Multistep step is 253 warp instructions (341 before): 88 on the float64 pipe,
+// 70 FMA, 43 ALU, 24 XU (float <-> float64 conversions); issue is 69 % busy,
 // the float64 and XU pipes about half, so issue and latency bound it.
 #include "boris32_common.cuh"
 #include "seg_common.cuh"

@@ -4,12 +4,12 @@
 // or both fields uniform (fixed steps).
 //
 // Measured on the device, against k_fixed64: dipole, MultistepBoris4(2), 1e6
-// protons x 1000 steps 31.7 -> 16.9 ms (443 instead of 733 warp instructions
-// per step, 243 instead of 358 of them on the float64 pipe, which is 71 %
+// protons x 1000 steps 31.7 -> 16.9 ms (447 instead of 733 warp instructions
+// per step, 244 instead of 358 of them on the float64 pipe, which is 72 %
 // busy: that pipe is the bound); uniform field, Boris, 1000 protons x 1e4
 // steps 13.5 -> 0.85 ms (one warp per sub-partition: the bound is the chain
 // of dependent operations, 166 cycles per step); dipole, AdaptiveBoris(0.1), 300001 protons
-// of at most 1000 steps 7.53 -> 4.28 ms.
+// of at most 1000 steps 7.53 -> 4.25 ms.
 #include "boris64_common.cuh"
 #include "seg_common.cuh"
 

@@ -410,7 +410,7 @@ __device__ __forceinline__ D3 multistep_rot64(D3 v, D3 E, D3 B, double q2m, doub
 
 // ---------------------------------------------------------------- updates of the segment kernels
 // E zero, B a dipole (FK_DIPOLE): the arithmetic of analytic_eval64 / boris_rot64 / multistep_rot64 with the
-// shared reciprocals of fdiv64.cuh and without the terms of a zero E: 237
+// shared reciprocals of fdiv64.cuh and without the terms of a zero E: 244
 // float64-pipe instructions per Multistep step instead of 358.  The float64
 // pipe (16 lanes per sub-partition) is what bounds these kernels.  They return
 // false, with nothing computed, where a denominator is outside the range of

@@ -37,11 +37,10 @@ __host__ __device__ __forceinline__ int gc_grid_mode(const DevFields& f) {
     return (ge || gb || quad) ? GM_GRID : GM_ANALYTIC;
 }
 
-//
 // A right-hand side class has the grid mode kGM, register caps for the two
 // drivers (threads), start(p), called once per particle, and kFast: it computes
 // in a restricted range and clears ok outside it, upon which the driver repeats
-// the step with RHS64 (step_general).
+// the step with RHS64 (rk4_general, dp5_general).
 template <int GM>
 struct RHS64 {
     static constexpr int kGM = GM, kRk4Bound = 256, kRk45Bound = 384;

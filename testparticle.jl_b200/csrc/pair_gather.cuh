@@ -1,7 +1,8 @@
 // pair_gather.cuh -- trilinear stencils gathered by pairs of lanes.
 //
 // A node of the interleaved table (E xyz0, B xyz0) or of one float64 field is 32
-// bytes, z is the tables' fastest axis, and a 128-byte line holds four nodes that are neighbours along z.  When
+// bytes, z is the tables' fastest axis, and a 128-byte line holds four nodes that are
+// neighbours along z.  When
 // every lane loads the 8 corners of its own particle, the 32 lanes of a load
 // instruction touch 32 different lines, and the L1 cache, which looks up one
 // line per clock, needs 8 x 32 clocks per warp and step: that bounded the

@@ -158,6 +158,8 @@ cudaError_t launch_table_sum(const float4* tab, int64_t nodes, int stride, int o
 // node-gradient table -> user layout out[3*k + c] (float64, scaled back by 2^G)
 cudaError_t launch_table_unpack(const float4* tab, int64_t nodes, int stride, int off, int G, double* out,
                                 cudaStream_t s);
+// the same for the E (off 0) or B (off 1) half of the interleaved table
+cudaError_t launch_eb_unpack(const float4* tab, const int32_t n[3], int off, int G, double* out, cudaStream_t s);
 
 // the kernel of a run that seg_config() accepts (boris_seg64.cu, boris_seg32.cu)
 const void* seg_kernel64(const BorisArgs& a, bool queue);
@@ -166,8 +168,6 @@ const void* seg_kernel32(const BorisArgs& a, bool queue);
 const void* grid_kernel64(const BorisArgs& a, bool queue);
 const void* gridb_kernel64(const BorisArgs& a, bool queue);  // B alone on one (gridb_config)
 const void* grid_kernel32(const BorisArgs& a, bool queue);
-// the same for the E (off 0) or B (off 1) half of the interleaved table
-cudaError_t launch_eb_unpack(const float4* tab, const int32_t n[3], int off, int G, double* out, cudaStream_t s);
 
 cudaError_t launch_boris_fp64(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s);
 cudaError_t launch_boris_fp32c(const BorisArgs& a, const LaunchCfg& c, cudaStream_t s);
@@ -215,9 +215,9 @@ cudaError_t cell_order(const double* u0, int64_t n, const DevField& g, void* tmp
                        int32_t** perm, cudaStream_t s);
 cudaError_t launch_pack_node_table(const void* src, int src_f64, int64_t nodes, void* dst,
                                    int dst_f64, int stride, int off, cudaStream_t s);
-// E and B data (both float64, or both float32) into the interleaved table
 // the same with z fastest (tri_node): the table of a trilinear uniform-Cartesian grid
 cudaError_t launch_pack_tri(const void* src, int src_f64, const int32_t n[3], void* dst, int dst_f64, cudaStream_t s);
+// E and B data (both float64, or both float32) into the interleaved table
 cudaError_t launch_pack_eb(const void* E, const void* B, int src_f64, const int32_t n[3], void* dst, cudaStream_t s);
 cudaError_t launch_pack_results(const double* t_in, const double* u_in, const int32_t* nsaved,
                                 const int64_t* offsets, int64_t n, int64_t nslots, int width,
