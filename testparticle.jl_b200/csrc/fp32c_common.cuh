@@ -593,9 +593,10 @@ __device__ __forceinline__ D3 cpos_d3(const CPos& p) {
             (double)p.hi[2] + (double)p.lo[2]};
 }
 
-// The contractions of this section are spelled out: a kernel that has the step in more
-// than one place (seg_common.cuh) must round it the same way in each, or an orbit
-// would depend on which lanes share its warp.
+// The contractions of this section are spelled out, in the form that the compiler gives
+// the plain expressions: a kernel that has the step in more than one place
+// (seg_common.cuh) must round it the same way in each, or an orbit would depend on which
+// lanes share its warp.
 __device__ __forceinline__ double dot_fma(D3 a, D3 b) { return fma(a.z, b.z, fma(a.x, b.x, __dmul_rn(a.y, b.y))); }
 __device__ __forceinline__ D3 cross_fma(D3 a, D3 b) {
     return {fma(a.y, b.z, -__dmul_rn(a.z, b.y)), fma(a.z, b.x, -__dmul_rn(a.x, b.z)),
@@ -663,7 +664,7 @@ __device__ __forceinline__ RotMixed rotation_mixed(D3 E, D3 B, double fac, int N
             e_corr = fmaf(-s2, 1.0f / 15.0f, -1.0f / 3.0f);
         }
         const double fd = f_N;
-        if (hasE) e = axpy(__dmul_rn((double)e_corr, dot_fma(e, t)), t, scale_rn(fd, e));
+        if (hasE) e = axpy(fd, e, scale_rn(__dmul_rn((double)e_corr, dot_fma(e, t)), t));
         t = scale_rn(fd, t);
         sd = __dmul_rn(__dmul_rn(fd, fd), sd);
         s = (float)sd;
@@ -694,7 +695,7 @@ __device__ __forceinline__ RotMixed rotation_mixed(D3 E, D3 B, double fac, int N
 }
 
 __device__ __forceinline__ D3 rotate_mixed(D3 v, const RotMixed& m, bool hasE) {
-    D3 dv = axpy(__dmul_rn(m.C3, dot_fma(v, m.t)), m.t, axpy(m.C2, cross_fma(v, m.t), scale_rn(m.C1, v)));
+    D3 dv = axpy(__dmul_rn(m.C3, dot_fma(v, m.t)), m.t, axpy(m.C1, v, scale_rn(m.C2, cross_fma(v, m.t))));
     if (hasE)
         dv = axpy(__dmul_rn(m.c6, dot_fma(m.e, m.t)), m.t, axpy(m.C3, cross_fma(m.e, m.t), axpy(m.C2, m.e, dv)));
     return {__dadd_rn(v.x, dv.x), __dadd_rn(v.y, dv.y), __dadd_rn(v.z, dv.z)};
