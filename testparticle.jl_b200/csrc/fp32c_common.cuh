@@ -98,11 +98,11 @@ struct AxF {
 __device__ __forceinline__ bool axis32(const DevField& g, int a, float hi, float lo, AxF& o) {
     const float kMagic = 12582912.0f;  // 1.5 * 2^23
     float d = hi - g.x0f[a];
-    float u = d * g.idxf[a];
+    float u = __fmul_rn(d, g.idxf[a]);
     float fl;
     int i;
     if (fabsf(u) < 4194304.0f) {
-        float tr = u + kMagic;
+        float tr = __fadd_rn(u, kMagic);
         i = __float_as_int(tr) - __float_as_int(kMagic);
         fl = tr - kMagic;
     } else {
@@ -110,15 +110,15 @@ __device__ __forceinline__ bool axis32(const DevField& g, int a, float hi, float
         i = (int)fl;
     }
     float rem = fmaf(-fl, g.dxf[a], d) + lo;
-    float f = rem * g.idxf[a];
+    float f = __fmul_rn(rem, g.idxf[a]);
     if (f < 0.0f) {
         fl -= 1.0f;
         i -= 1;
-        f += 1.0f;
+        f = __fadd_rn(f, 1.0f);
     } else if (f >= 1.0f) {
         fl += 1.0f;
         i += 1;
-        f -= 1.0f;
+        f = __fadd_rn(f, -1.0f);
     }
     int na = g.n[a];
     if (g.bc == TP_BC_PERIODIC) {
@@ -134,7 +134,7 @@ __device__ __forceinline__ bool axis32(const DevField& g, int a, float hi, float
         o.ds = g.idxf[a];
         return true;
     }
-    float uc = fl + f;
+    float uc = __fadd_rn(fl, f);
     float umax = (float)(na - 1);
     o.ds = g.idxf[a];
     if (g.bc == TP_BC_CLAMP) {

@@ -42,14 +42,16 @@ def _setup(tp, field, n):
     u0 = np.concatenate([DX * np.array(shape)[:, None] * rng.uniform(0.1, 0.9, (3, n)), 2.0e5 * rng.normal(size=(3, n))])
     if field == "b64":
         return tp.ZeroField(), _grid(tp, shape, np.float64, tp.FillExtrap()), u0, dt
-    kind, order = np.float32 if field == "eb32" else np.float64, 3 if field == "cubic64" else 1
-    return [_grid(tp, shape, kind, tp.WrapExtrap(), s, scale, order) for s, scale in ((5, 4.0e5), (4, 1.0))] + [u0, dt]
+    kind, order = np.float32 if field.startswith("eb32") else np.float64, 3 if field == "cubic64" else 1
+    bc = {"eb32clamp": tp.ClampExtrap(), "eb32fill": tp.FillExtrap()}.get(field, tp.WrapExtrap())
+    return [_grid(tp, shape, kind, bc, s, scale, order) for s, scale in ((5, 4.0e5), (4, 1.0))] + [u0, dt]
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32c"])
 @pytest.mark.parametrize("alg", ["boris", "ms4"])
 @pytest.mark.parametrize("field,n,every", [("uniform", 3000, 3), ("dipole", 3000, 3), ("dipole", 200000, 1), ("eb32", 3000, 40),
-                                           ("eb32", 70000, 2), ("eb32", 70000, 20), ("b64", 3000, 3), ("eb64", 70000, 20), ("cubic64", 70000, 20)])
+                                           ("eb32", 70000, 2), ("eb32", 70000, 20), ("eb32clamp", 200000, 20),
+                                           ("eb32clamp", 70000, 2), ("eb32fill", 70000, 2), ("b64", 3000, 3), ("eb64", 70000, 20), ("cubic64", 70000, 20)])
 def test_orbits_alone_and_together(tp, field, n, every, alg, precision):
     E, B, u0, dt = _setup(tp, field, n)
     a = {"boris": tp.Boris(), "ms4": tp.MultistepBoris4(2)}[alg]
